@@ -133,6 +133,7 @@ def _load():
         "iga_lmode_apply": ([i32, i32, C.POINTER(iga_factor), i64, vp, vp, vp, vp, vp], i32),
         "iga_pointwise_scale": ([i32, i64, i64, vp, i64, vp, vp, i32, vp], i32),
         "iga_axpby": ([i32, i64, C.c_double, vp, C.c_double, vp, vp], i32),
+        "iga_mf_resident": ([C.POINTER(iga_mf_plan), i32, C.POINTER(C.c_int32)], i32),
         "iga_mf_layout": ([C.POINTER(iga_mf_plan), i32, C.POINTER(C.c_int64), vp], i32),
         "iga_mf_pack": ([C.POINTER(iga_mf_plan), i32, vp, i64, i32, vp, vp], i32),
         "iga_mf_table": ([C.POINTER(iga_mf_plan), i32, C.POINTER(C.c_int64), vp, vp], i32),
@@ -245,6 +246,7 @@ def exported_symbols():
         "iga_pointwise_scale",
         "iga_axpby",
         "iga_mf_layout",
+        "iga_mf_resident",
         "iga_mf_pack",
         "iga_mf_table",
         "iga_mf_matvec",

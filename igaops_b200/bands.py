@@ -234,6 +234,12 @@ class RuleBands:
     def rwidth(self) -> int:
         return self.testR[2]
 
+    def group_count(self, most: int) -> int:
+        """Groups of at most `most` points between moves of either window."""
+        moves = (np.diff(self.trial[0]) != 0) | (np.diff(self.testT[0]) != 0)
+        edges = np.concatenate([[0], np.flatnonzero(moves) + 1, [self.nq]])
+        return int(np.sum(-(-np.diff(edges) // most)))
+
     def device(self, dtype: torch.dtype, W: int, RW: int):
         key = (dtype, W, RW)
         hit = self._dev.get(key)

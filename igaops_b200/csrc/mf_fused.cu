@@ -3,6 +3,7 @@
 #include <vector>
 
 #include "mf_fused.cuh"
+#include "mf_warp.cuh"
 
 namespace iga {
 
@@ -47,7 +48,20 @@ static iga_status check_plan(const iga_mf_plan* p) {
   return IGA_OK;
 }
 
+// The face selects the 3D kernel: 8 x 8 is the warp-per-tile kernel, whose
+// chunks hold the whole tile (padding pencils zero).
+static bool warp_face(const iga_mf_plan* p) {
+  return p->ndim == 3 && p->face[0] == kWarpFace && p->face[1] == kWarpFace;
+}
+
 static int64_t layout_elems(const iga_mf_plan* p, int dtype, int64_t* tile_off) {
+  if (warp_face(p)) {
+    const int64_t tiles = ceil_div(p->nq[0], p->face[0]) * ceil_div(p->nq[1], kWarpFace);
+    // [group][tile][point][stream][pencil]: a tile has no offset of its own
+    if (tile_off)
+      for (int64_t t = 0; t < tiles; ++t) tile_off[t] = 0;
+    return tiles * p->nq[2] * p->nstream * kWarpTile;
+  }
   const int FX = p->face[0];
   const int FY = p->ndim == 3 ? p->face[1] : 1;
   const int tiles1 = (int)ceil_div(p->nq[0], FX);
@@ -121,6 +135,133 @@ __global__ void __launch_bounds__(256) mf_pack3_pm_kernel(int nq1, int nq2, int 
   Tout* dst = packed + tile_off[tile] + (int64_t)q3 * chunk_stride_elems<Tout>(S, w1, w2) +
               ((int64_t)l2 * w1 + l1) * S;
   for (int s = 0; s < S; ++s) dst[s] = (Tout)coefs[(int64_t)rows.r[s] * ld + q];
+}
+
+// pack for the warp-per-tile kernel, [group][tile][point][stream][pencil]: one
+// CTA per (row of tiles, q3); a warp walks one row of points (coalesced reads)
+// and writes its 8-point pieces into the row's tiles, zeros beyond the grid.
+template <typename Tin, typename Tout>
+__global__ void __launch_bounds__(256)
+    mf_pack_warp_kernel(int nq1, int nq2, int nq3, int S, int tiles1, int tiles2,
+                        const int32_t* __restrict__ groups, SrcRows rows,
+                        const Tin* __restrict__ coefs, int64_t ld, Tout* __restrict__ packed) {
+  const int t2 = blockIdx.x, q3 = blockIdx.y;
+  int lo = 0, hi = __ldg(groups);  // the group of q3
+  while (hi - lo > 1) {
+    const int mid = (lo + hi) >> 1;
+    if ((__ldg(groups + 1 + mid) >> 2) <= q3) lo = mid;
+    else hi = mid;
+  }
+  const int qg = __ldg(groups + 1 + lo) >> 2, np = (__ldg(groups + 2 + lo) >> 2) - qg;
+  const int64_t chunk = (int64_t)S * kWarpTile, tstride = np * chunk;
+  Tout* base = packed + ((int64_t)qg * tiles1 * tiles2 + (int64_t)t2 * tiles1 * np + (q3 - qg)) * chunk;
+  for (int row = threadIdx.x >> 5; row < S * kWarpFace; row += 8) {
+    const int s = row / kWarpFace, l2 = row % kWarpFace;
+    const int q2 = t2 * kWarpFace + l2;
+    const Tin* src = coefs + (int64_t)rows.r[s] * ld + ((int64_t)q3 * nq2 + q2) * nq1;
+    Tout* dst = base + s * kWarpTile + l2 * kWarpFace;
+    for (int q1 = threadIdx.x & 31; q1 < tiles1 * kWarpFace; q1 += 32)
+      dst[(q1 / kWarpFace) * tstride + q1 % kWarpFace] =
+          (q1 < nq1 && q2 < nq2) ? (Tout)src[q1] : Tout(0);
+  }
+}
+
+// step rows of the warp-per-tile kernel: the pattern's value groups (src)
+template <typename T>
+struct RowSrc {
+  const T* p[4];
+  int n;
+};
+template <typename T>
+__global__ void mf_table_warp_kernel(int nq, int W, RowSrc<T> src, T* __restrict__ table) {
+  const int G = step_group<T>(W), rlen = src.n * G;
+  const int64_t total = (int64_t)nq * rlen;
+  for (int64_t idx = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; idx < total;
+       idx += (int64_t)gridDim.x * blockDim.x) {
+    const int q = (int)(idx / rlen), j = (int)(idx - (int64_t)q * rlen);
+    const int grp = j / G, k = j - grp * G;
+    table[idx] = k < W ? src.p[grp][(int64_t)q * W + k] : T(0);
+  }
+}
+
+// group list behind the step rows (see group_list_offset): runs of points
+// between window moves, cut into pieces of at most kGroupPts points of nearly
+// equal size; one CTA, thread q0 + t decides for point q whether a group starts
+// there, a running prefix sum numbers them
+__global__ void __launch_bounds__(256) mf_groups_kernel(int nq, const int32_t* __restrict__ ts,
+                                                        const int32_t* __restrict__ ws,
+                                                        int32_t* __restrict__ list) {
+  __shared__ int s_cnt[256];
+  auto moves = [&](int q) {
+    return q <= 0 ? 0 : (ts[q] != ts[q - 1] ? 1 : 0) | (ws[q] != ws[q - 1] ? 2 : 0);
+  };
+  int base = 0;
+  for (int q0 = 0; q0 < nq; q0 += 256) {
+    const int q = q0 + threadIdx.x;
+    bool start = false;
+    if (q < nq) {
+      int lo = q, hi = q + 1;  // the run [lo, hi) of q
+      while (lo > 0 && !moves(lo)) --lo;
+      while (hi < nq && !moves(hi)) ++hi;
+      const int len = hi - lo, np = (len + kGroupPts - 1) / kGroupPts;
+      for (int k = 0; k < np; ++k) start |= q == lo + (int)((int64_t)len * k / np);
+    }
+    s_cnt[threadIdx.x] = start;
+    __syncthreads();
+    int rank = 0, total = 0;
+    for (int t = 0; t < 256; ++t) {
+      rank += t < (int)threadIdx.x ? s_cnt[t] : 0;
+      total += s_cnt[t];
+    }
+    if (start) list[1 + base + rank] = q << 2 | moves(q);
+    base += total;
+    __syncthreads();
+  }
+  if (threadIdx.x == 0) {
+    list[0] = base;
+    list[1 + base] = nq << 2;
+  }
+}
+
+// derivative orders of the streamed direction that an operator reads: bit 0 /
+// bit 1 = order 0 / 1 of the trial bands, bit 2 / 3 of the test bands
+static int last_orders(const iga_mf_plan* p) {
+  if (p->spacetime) return (1 << p->time_trial) | (4 << p->time_test);
+  const bool tg = p->op == IGA_OP_STIFF || p->op == IGA_OP_U_GRADV;
+  const bool wg = p->op == IGA_OP_STIFF || p->op == IGA_OP_GRADU_V;
+  return (tg ? 3 : 1) | (wg ? 12 : 4);
+}
+
+// byte offset of the group list in the step table
+static int64_t group_list_bytes(const iga_mf_plan* p, int dtype) {
+  const int o = last_orders(p), n = (o & 1) + (o >> 1 & 1) + (o >> 2 & 1) + (o >> 3);
+  const int nq = p->nq[p->ndim - 1];
+  return dtype == IGA_F64 ? group_list_offset<double>(nq, n * step_group<double>(p->width))
+                          : group_list_offset<float>(nq, n * step_group<float>(p->width));
+}
+
+template <typename T>
+static iga_status table_warp(const iga_mf_plan* p, int64_t* elems, void* table, cudaStream_t st) {
+  const int o = last_orders(p), last = p->ndim - 1;
+  RowSrc<T> src;
+  src.n = 0;
+  if (o & 1) src.p[src.n++] = (const T*)p->trial[last].vals;
+  if (o & 2) src.p[src.n++] = (const T*)p->trial_d1[last];
+  if (o & 4) src.p[src.n++] = (const T*)p->testT[last].vals;
+  if (o & 8) src.p[src.n++] = (const T*)p->testT_d1[last];
+  const int rlen = src.n * step_group<T>(p->width), nq = p->nq[last];
+  const int64_t off = group_list_offset<T>(nq, rlen);
+  // at most one group per point, the count and the end mark
+  *elems = (off + 4 * ((int64_t)nq + 2) + (int64_t)sizeof(T) - 1) / (int64_t)sizeof(T);
+  if (!table) return IGA_OK;
+  for (int i = 0; i < src.n; ++i) IGA_CHECK_ARG(src.p[i], "band values missing");
+  IGA_CHECK_ARG(p->trial[last].start && p->testT[last].start, "band starts missing");
+  const unsigned g = (unsigned)std::min<int64_t>(ceil_div((int64_t)nq * rlen, 256), 148 * 8);
+  mf_table_warp_kernel<T><<<g, 256, 0, st>>>(nq, p->width, src, (T*)table);
+  mf_groups_kernel<<<1, 256, 0, st>>>(nq, p->trial[last].start, p->testT[last].start,
+                                      (int32_t*)((char*)table + off));
+  IGA_LAUNCH_CHECK();
+  return IGA_OK;
 }
 
 // step table rows of the last direction: B0, B1, W0T, W1T (W each), starts
@@ -227,8 +368,16 @@ iga_status launch_dispatch<float>(const FusedArgs<float>& a, const LaunchInfo& l
 template <typename T>
 static size_t batch_smem(const iga_mf_plan* p, int rlen) {
   const int W = p->width, RW = p->rwidth;
-  auto f = [&](auto pat) {
+  auto f = [&](auto pat) -> size_t {
     using P = decltype(pat);
+    if (warp_face(p)) {
+      switch (W) {
+        case 3: return WarpSmem<T, P, 3>::total;
+        case 4: return WarpSmem<T, P, 4>::total;
+        case 5: return WarpSmem<T, P, 5>::total;
+        default: return WarpSmem<T, P, 6>::total;
+      }
+    }
     return mf3d_smem_bytes<T, P>(kFace3X, kFace3Y, W, RW, rlen, p->cmax[0], p->cmax[1],
                                  p->dmax[0], p->dmax[1]);
   };
@@ -265,8 +414,12 @@ static iga_status batch_prepare(const iga_mf_plan* plans, int npatch, const void
     if (rc) return rc;
     IGA_CHECK_ARG(p->ndim == 3 && !p->spacetime, "patch %d: multi-patch matvec covers 3D space operators", i);
     IGA_CHECK_ARG(p->op == p0.op && p->sym == p0.sym && p->width == p0.width &&
-                      p->face[0] == kFace3X && p->face[1] == kFace3Y,
+                      p->face[0] == p0.face[0] && p->face[1] == p0.face[1] &&
+                      (warp_face(p) || (p->face[0] == kFace3X && p->face[1] == kFace3Y)),
                   "patch %d: operator, symmetry, band width and face must match patch 0", i);
+    const int range = p->width + kWarpFace - 1;
+    IGA_CHECK_ARG(!warp_face(p) || std::max({p->cmax[0], p->cmax[1], p->dmax[0], p->dmax[1]}) <= range,
+                  "patch %d: control ranges of a tile exceed %d", i, range);
     IGA_CHECK_ARG(packed[i] && ((uintptr_t)packed[i] & 15) == 0 && p->step_table,
                   "patch %d: packed coefficients (16-byte aligned) and step table required", i);
     fill_args<T>(args[i], p, packed[i], nullptr, nullptr);
@@ -366,6 +519,7 @@ iga_status iga_mf_batch_matvec(const iga_mf_plan* plan0, int dtype, int npatch, 
   b.op = plan0->op;
   b.sym = plan0->sym;
   b.W = plan0->width;
+  b.warp = warp_face(plan0);
   b.npatch = npatch;
   b.total_ctas = total_ctas;
   b.smem = (size_t)smem_bytes;
@@ -382,6 +536,16 @@ iga_status iga_mf_batch_matvec(const iga_mf_plan* plan0, int dtype, int npatch, 
   if (dtype == IGA_F32) return batch_dispatch<float>(b, (const float*)x, (float*)y);
   set_error("dtype %d not supported", dtype);
   return IGA_ERR_UNSUPPORTED;
+}
+
+iga_status iga_mf_resident(const iga_mf_plan* plan, int dtype, int32_t* ctas) {
+  clear_error();
+  iga_status rc = check_plan(plan);
+  if (rc) return rc;
+  IGA_CHECK_ARG(dtype == IGA_F64 || dtype == IGA_F32, "dtype %d not supported", dtype);
+  IGA_CHECK_ARG(ctas, "null ctas");
+  *ctas = warp_face(plan) ? warp_resident(dtype == IGA_F64, plan->nstream, plan->width) : 0;
+  return IGA_OK;
 }
 
 iga_status iga_mf_layout(const iga_mf_plan* plan, int dtype, int64_t* elems,
@@ -402,6 +566,9 @@ iga_status iga_mf_table(const iga_mf_plan* plan, int dtype, int64_t* elems, void
   if (rc) return rc;
   IGA_CHECK_ARG(elems, "null elems");
   IGA_CHECK_ARG(dtype == IGA_F64 || dtype == IGA_F32, "dtype %d not supported", dtype);
+  if (warp_face(plan))
+    return dtype == IGA_F64 ? table_warp<double>(plan, elems, table, as_stream(stream))
+                            : table_warp<float>(plan, elems, table, as_stream(stream));
   const int last = plan->ndim - 1;
   const int W = plan->width;
   const int nq = plan->nq[last];
@@ -444,10 +611,30 @@ iga_status iga_mf_pack(const iga_mf_plan* plan, int dtype_in, const void* coefs,
   cudaStream_t st = as_stream(stream);
   const int64_t elems = layout_elems(plan, dtype_out, nullptr);
   const size_t esz = dtype_out == IGA_F64 ? 8 : 4;
-  IGA_CUDA_TRY(cudaMemsetAsync(packed, 0, (size_t)elems * esz, st));
   int64_t Nq = 1;
   for (int d = 0; d < plan->ndim; ++d) Nq *= plan->nq[d];
   IGA_CHECK_ARG(ld >= Nq, "ld %lld smaller than Nq %lld", (long long)ld, (long long)Nq);
+  if (warp_face(plan)) {
+    const int nq3 = plan->nq[2], tiles1 = (int)ceil_div(plan->nq[0], plan->face[0]);
+    IGA_CHECK_ARG(nq3 <= 65535, "streamed direction of %d points exceeds the grid", nq3);
+    const int tiles2 = (int)ceil_div(plan->nq[1], kWarpFace);
+    IGA_CHECK_ARG(plan->step_table, "face (8, 8) packs by the step table's groups (iga_mf_table)");
+    const dim3 grid((unsigned)tiles2, (unsigned)nq3);
+    const int32_t* groups =
+        (const int32_t*)((const char*)plan->step_table + group_list_bytes(plan, dtype_out));
+#define IGA_PACK(TI, TO)                                                                     \
+  mf_pack_warp_kernel<TI, TO><<<grid, 256, 0, st>>>(plan->nq[0], plan->nq[1], nq3, S, tiles1, \
+                                                    tiles2, groups, rows, (const TI*)coefs,  \
+                                                    ld, (TO*)packed)
+    if (dtype_in == IGA_F64 && dtype_out == IGA_F64) IGA_PACK(double, double);
+    else if (dtype_in == IGA_F64 && dtype_out == IGA_F32) IGA_PACK(double, float);
+    else if (dtype_in == IGA_F32 && dtype_out == IGA_F64) IGA_PACK(float, double);
+    else IGA_PACK(float, float);
+#undef IGA_PACK
+    IGA_LAUNCH_CHECK();
+    return IGA_OK;
+  }
+  IGA_CUDA_TRY(cudaMemsetAsync(packed, 0, (size_t)elems * esz, st));
   int64_t blocks = ceil_div(Nq * S, 256);
   if (blocks > 148 * 64) blocks = 148 * 64;
   const int nq3 = plan->ndim == 3 ? plan->nq[2] : 1;

@@ -1337,6 +1337,7 @@ struct LaunchInfo {
 // Multi-patch 3D launch (all patches share op, symmetry and band width).
 struct BatchLaunch {
   int op, sym, W;
+  bool warp;  // 8 x 8 face: the warp-per-tile kernel
   int npatch, total_ctas;
   size_t smem;
   const void* args;     // device FusedArgs<T>[npatch]

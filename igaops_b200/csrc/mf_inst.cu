@@ -2,6 +2,7 @@
 // this file once per (IGA_INST_D, IGA_INST_T, IGA_INST_W) so that the many
 // template instances build in parallel.
 #include "mf_fused.cuh"
+#include "mf_warp.cuh"
 
 #ifndef IGA_INST_D
 #define IGA_INST_D 3
@@ -16,6 +17,22 @@ template <typename T, int D, int W, class P>
 static iga_status launch_pat(const FusedArgs<T>& a, const LaunchInfo& li) {
   const dim3 grid((unsigned)(a.tiles1 * a.tiles2 * a.nseg), (unsigned)li.ncols);
   if constexpr (D == 3) {
+    if (li.FX == kWarpFace && li.FY == kWarpFace) {
+      if (!a.step_table) {
+        set_error("3D fused kernel needs the step table of the plan (iga_mf_table)");
+        return IGA_ERR_INVALID_ARG;
+      }
+      using L = WarpSmem<T, P, W>;
+      if (std::max({a.cmax1, a.cmax2, a.dmax1, a.dmax2}) > L::range) {
+        set_error("control ranges %d/%d/%d/%d of a tile exceed %d", a.cmax1, a.cmax2, a.dmax1,
+                  a.dmax2, L::range);
+        return IGA_ERR_UNSUPPORTED;
+      }
+      static_assert(L::total <= 48 * 1024, "shared memory of a CTA (no opt-in)");
+      mfw_kernel<T, W, P><<<grid, 32, L::total, li.stream>>>(a);
+      IGA_LAUNCH_CHECK();
+      return IGA_OK;
+    }
     constexpr int FX = kFace3X, FY = kFace3Y;
     if (li.FX != FX || li.FY != FY) {
       set_error("3D fused kernels are compiled for a %dx%d face, plan has %dx%d", FX, FY, li.FX,
@@ -99,6 +116,12 @@ static iga_status launch_pat_batch(const BatchLaunch& b, const T* x, T* y) {
   if (b.smem > 227 * 1024) {
     set_error("multi-patch fused kernel needs %zu bytes of shared memory", b.smem);
     return IGA_ERR_UNSUPPORTED;
+  }
+  if (b.warp) {
+    mfw_batch_kernel<T, W, P><<<(unsigned)b.total_ctas, 32, b.smem, b.stream>>>(
+        (const FusedArgs<T>*)b.args, b.cta0, b.npatch, b.offs, x, y, b.skip);
+    IGA_LAUNCH_CHECK();
+    return IGA_OK;
   }
   auto kern = mf3d_batch_kernel<T, FX, FY, W, P>;
   static size_t configured = 48 * 1024;

@@ -160,9 +160,12 @@ def _src_rows(ndim, op, st, sym, lead2: int):
     return rows
 
 
-FACE3 = (16, 8)
+# 3D tiles are 8 x 8, one warp each (csrc/mf_warp.cuh): faster than the 16 x 8
+# CTA-per-tile kernel at every degree, type and size timed (8^3 to 128^3)
+FACE3 = (8, 8)
 FACE2 = (128,)
 _SM_COUNT = 148
+_GROUP_POINTS = 3  # points per group of the 3D kernel (kGroupPts)
 
 
 class FusedPlan:
@@ -205,15 +208,10 @@ class FusedPlan:
         tiles1 = -(-self.nq[0] // face[0])
         tiles2 = -(-self.nq[1] // face[1]) if ndim == 3 else 1
         nlast = self.nq[-1]
-        if nseg is None:
-            # about 12 CTAs per SM (one resident CTA per SM in 3D), segments of
-            # at least 48 points so window warm-up and flush stay amortised
-            target = _SM_COUNT * 12
-            nseg = max(1, min(-(-target // (tiles1 * tiles2)), nlast // 48))
-        nseg = max(1, min(int(nseg), nlast))
-        P.nseg = nseg
-        self.nseg = nseg
-        self.units = tiles1 * tiles2 * nseg
+        # 3D: groups of points between window moves, the unit segments are cut in
+        self.groups = rbs[-1].group_count(_GROUP_POINTS) if ndim == 3 else 0
+        self.tiles = tiles1 * tiles2
+        P.nseg = 1
         # tile ranges for shared-memory sizing
         cmax, dmax = [1, 1], [1, 1]
         for d in range(min(ndim - 1, 2)):
@@ -236,6 +234,23 @@ class FusedPlan:
             P.testR_d1[d] = testR.vals[1].data_ptr()
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         P.status = self.status.data_ptr()
+        self.resident = 0
+        if ndim == 3:
+            res = ctypes.c_int32(0)
+            _lib.check(_lib.LIB.iga_mf_resident(ctypes.byref(P), iga_dtype(dtype),
+                                                ctypes.byref(res)))
+            self.resident = int(res.value)
+        if nseg is None:
+            if ndim == 3:
+                nseg = self.predicted_nseg()[0]
+            else:
+                # about 12 CTAs per SM, segments of at least 48 points so window
+                # warm-up and flush stay amortised
+                nseg = max(1, min(-(-_SM_COUNT * 12 // self.tiles), nlast // 48))
+        nseg = max(1, min(int(nseg), nlast))
+        P.nseg = nseg
+        self.nseg = nseg
+        self.units = self.tiles * nseg
         # packed layout
         off = np.zeros(tiles1 * tiles2, dtype=np.int64)
         elems = ctypes.c_int64(0)
@@ -256,13 +271,30 @@ class FusedPlan:
         P.step_table = self.step_table.data_ptr()
         self.P = P
 
+    def predicted_nseg(self, most: int = 64):
+        """Segment counts of the 3D kernel, the one that should run fastest first.
+
+        Units (tile x segment, one warp each) run in waves of 148 x resident
+        warps.  A unit costs its share of the groups plus a fixed part (set-up,
+        W plane productions and flushes), about five groups; a warp with the SM
+        to itself takes a group in 1 / 1.6 of the time it takes among all
+        resident ones (3D p3 128^3 mass: 1.03 against 1.6 us).  The last,
+        partly filled wave is charged at its own residency."""
+        full = _SM_COUNT * max(self.resident, 3)
+
+        def cost(ns):
+            units = self.tiles * ns
+            waves, rest = divmod(units, full)
+            return (1.6 * waves + (1 + 0.6 * rest / full if rest else 0)) * (self.groups / ns + 5)
+
+        return sorted(range(1, max(1, min(most, self.groups // 2)) + 1), key=cost)
+
     def set_nseg(self, nseg: int):
         """Segments of the streamed direction (work units = tiles x nseg)."""
         nseg = max(1, min(int(nseg), self.nq[-1]))
-        tiles = self.units // self.nseg
         self.P.nseg = nseg
         self.nseg = nseg
-        self.units = tiles * nseg
+        self.units = self.tiles * nseg
 
     def set_src_rows(self, lead2: int):
         rows = _src_rows(self.ndim, self.op, self.st, self.sym, lead2)

@@ -4,13 +4,13 @@ Two choices, both timed on the operator's own packed data (CUDA events,
 best of a few launches) and kept per problem shape in a process-wide cache,
 optionally persisted as JSON (``IGAOPS_B200_TUNE`` names the file):
 
-* the tiling of the 3D work: the pencil kernel's (16 x 8 face tile,
-  segment of the streamed direction) units or the tensor-core kernel's
+* the tiling of the 3D work: the pencil kernel's (8 x 8 face tile, segment
+  of the streamed direction) units, one warp each, or the tensor-core kernel's
   16 x 8 x 16 point tiles, one persistent CTA per SM (``choose_kernel``;
   the two pack the coefficients differently, so the candidate is packed
   once for the timing and kept if it wins);
 * for the pencil kernel, the number of segments ``nseg``, which trades CTA
-  count (filling 148 SMs x 3 resident CTAs) against per-CTA pipeline
+  unit count (filling 148 SMs x the resident warps) against per-unit
   warm-up and halo work (``tune_nseg``; the packed layout does not depend on
   ``nseg``, so tuning re-launches the same data with a different plan field).
 """
@@ -64,13 +64,9 @@ def shape_key(plan) -> str:
 
 
 def candidates(plan) -> Iterable[int]:
-    nlast = plan.nq[-1]
-    tiles = plan.units // max(plan.nseg, 1)
-    out = {1, 2, 3, 4, 6, 8, 12, 16}
-    # enough CTAs for about 3 resident CTAs x 148 SMs x k waves
-    for k in (1, 2, 4):
-        out.add(-(-444 * k // max(tiles, 1)))
-    return sorted(n for n in out if 1 <= n <= max(1, nlast // 8))
+    # the counts the wave model ranks first (the best of a sweep of 1 .. 24 was
+    # among its first four for every operator timed)
+    return sorted(plan.predicted_nseg()[:4])
 
 
 def tune_nseg(plan, packed: torch.Tensor, x: torch.Tensor, y: torch.Tensor,
@@ -99,6 +95,11 @@ def tune_nseg(plan, packed: torch.Tensor, x: torch.Tensor, y: torch.Tensor,
         times[ns] = best
     plan.check_status()
     win = min(times, key=times.get)
+    # within the timing's noise the wave model's choice stands, so that the same
+    # operator gets the same launch shape (and rounding) in every process
+    model = plan.predicted_nseg()[0]
+    if times.get(model, float("inf")) <= max(1.02 * times[win], times[win] + 1.5e-3):
+        win = model
     plan.set_nseg(win)
     _CACHE[key] = win
     _save()
