@@ -8,6 +8,7 @@
 #include <string.h>
 
 #include "common.cuh"
+#include "dense_mode.cuh"
 
 namespace iga {
 
@@ -152,6 +153,12 @@ static iga_status mode_product_t(const iga_factor* M, int64_t outer, int64_t inn
   }
   IGA_CHECK_ARG(M->kind == 1 && M->dense, "dense factor has null data");
   const T* D = (const T*)M->dense;
+  if (dense_fits(rows, cols, outer * inner)) {
+    DenseMode<T> p = dense_compact<T>(D, M->ld_row, M->ld_col, rows, cols, outer, inner, x, y);
+    p.accumulate = accumulate;
+    return launch_dense_mode<T>(p, false, false, st);
+  }
+  // contracted extents beyond the shared-memory staging of the dense kernel
   if (inner >= 16) {
     // per o: C(rows x inner) = M(rows x cols) X_o(cols x inner)
     IGA_CHECK_ARG(outer <= 65535, "outer %lld too large", (long long)outer);
