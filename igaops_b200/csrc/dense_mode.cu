@@ -59,41 +59,51 @@ __global__ void __launch_bounds__(kDenseThreads) dense_mode_kernel(const __grid_
 
   // the next product may set itself up; it waits before it reads this output
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // A: lanes along the unit stride of the factor, zeros in the padding
+  constexpr int NW = kDenseThreads / 32;
+  // A: lanes along the unit stride of the factor (U: rows; U^T: 8 rows x 4
+  // columns per warp, 64-byte reads and conflict-free stores), zero padding
   if (p.ldc == 1) {
-    for (int r = warp; r < ar; r += kDenseThreads / 32)
-      for (int c = lane; c < kp; c += 32) {
-        if (r < mr && c < K) stage_elem(As + r * lda + c, p.A + (int64_t)(r_lo + r) * p.ldr + c);
-        else As[r * lda + c] = 0.0;
-      }
+    for (int r = warp; r < mr; r += NW) {
+      const T* src = p.A + (int64_t)(r_lo + r) * p.ldr;
+      double* dst = As + r * lda;
+#pragma unroll 4
+      for (int c = lane; c < K; c += 32) stage_elem(dst + c, src + c);
+    }
   } else {
-    // 8 (r) x 4 (c) per warp: 64-byte reads, conflict-free stores
-    for (int c = warp * 4 + tq; c < kp; c += kDenseThreads / 8)
-      for (int r = gq; r < ar; r += 8) {
-        if (r < mr && c < K)
-          stage_elem(As + r * lda + c, p.A + (int64_t)(r_lo + r) * p.ldr + (int64_t)c * p.ldc);
-        else As[r * lda + c] = 0.0;
-      }
+    for (int c = warp * 4 + tq; c < K; c += 4 * NW) {
+      const T* src = p.A + (int64_t)r_lo * p.ldr + (int64_t)c * p.ldc;
+      double* dst = As + c;
+#pragma unroll 4
+      for (int r = gq; r < mr; r += 8) stage_elem(dst + r * lda, src + (int64_t)r * p.ldr);
+    }
   }
+  for (int r = tid; r < ar; r += kDenseThreads)
+    for (int c = r < mr ? K : 0; c < kp; ++c) As[r * lda + c] = 0.0;
+  // X tile [c][n]; padding rows and columns zero
+  for (int e = tid; e < (xr - K) * BN; e += kDenseThreads) Xs[(K + e / BN) * LDX + e % BN] = 0.0;
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  // X tile [c][n]
   if (p.xc == 1) {  // the contracted mode is contiguous: 8 (c) x 4 (n) per warp
-    const int nl = lane >> 3, cl = lane & 7;
-    for (int n = warp * 4 + nl; n < BN; n += kDenseThreads / 8) {
+    for (int n = warp * 4 + (lane >> 3); n < BN; n += 4 * NW) {
       const uint32_t g = (uint32_t)n_lo + n;
-      const T* src = p.x + (n < bn ? (int64_t)(g / (uint32_t)p.xlo) * p.xhi + (int64_t)(g % (uint32_t)p.xlo) * p.xls : 0);
-      for (int c = cl; c < xr; c += 8) {
-        if (n < bn && c < K) stage_elem(Xs + c * LDX + n, src + c);
-        else Xs[c * LDX + n] = 0.0;
+      const T* src = p.x + (int64_t)(g / (uint32_t)p.xlo) * p.xhi + (int64_t)(g % (uint32_t)p.xlo) * p.xls;
+      double* dst = Xs + n;
+      if (n < bn) {
+#pragma unroll 4
+        for (int c = lane & 7; c < K; c += 8) stage_elem(dst + c * LDX, src + c);
+      } else {
+        for (int c = lane & 7; c < K; c += 8) dst[c * LDX] = 0.0;
       }
     }
   } else {
     const int n = tid % BN;
     const uint32_t g = (uint32_t)n_lo + n;
-    const T* src = p.x + (n < bn ? (int64_t)(g / (uint32_t)p.xlo) * p.xhi + (int64_t)(g % (uint32_t)p.xlo) * p.xls : 0);
-    for (int c = tid / BN; c < xr; c += kDenseThreads / BN) {
-      if (n < bn && c < K) stage_elem(Xs + c * LDX + n, src + c * p.xc);
-      else Xs[c * LDX + n] = 0.0;
+    const T* src = p.x + (int64_t)(g / (uint32_t)p.xlo) * p.xhi + (int64_t)(g % (uint32_t)p.xlo) * p.xls;
+    double* dst = Xs + n;
+    if (n < bn) {
+#pragma unroll 4
+      for (int c = tid / BN; c < K; c += kDenseThreads / BN) stage_elem(dst + c * LDX, src + c * p.xc);
+    } else {
+      for (int c = tid / BN; c < K; c += kDenseThreads / BN) dst[c * LDX] = 0.0;
     }
   }
   if constexpr (sizeof(T) == 8) asm volatile("cp.async.wait_all;" ::: "memory");

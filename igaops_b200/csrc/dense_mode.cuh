@@ -39,7 +39,9 @@ struct DenseMode {
   int32_t mb;           // rows per CTA
 };
 
-constexpr int kDenseThreads = 256;
+// 16 warps: the staging of the operands, instruction-bound, takes as long as the
+// products with 8 (96^3 p3 apply 86 us, with 16 warps 72)
+constexpr int kDenseThreads = 512;
 constexpr int kDenseMax = 384;  // largest contracted extent
 
 __host__ __device__ inline int dense_ld(int n) {  // smallest stride >= n, 4 mod 8
