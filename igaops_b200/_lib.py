@@ -142,6 +142,7 @@ def _load():
         "iga_mft_smem_bytes": ([C.POINTER(iga_mft_plan), C.POINTER(C.c_int64)], i32),
         "iga_mft_matvec": ([C.POINTER(iga_mft_plan), vp, i64, vp, vp, vp], i32),
         "iga_geometry_pointwise": ([i32, i32, i64, vp, vp, vp, vp, vp, vp], i32),
+        "iga_geometry_coefficients": ([C.POINTER(iga_mf_plan), vp, vp, vp, vp, vp], i32),
         "iga_nurbs_coefficients": ([i32, i32, i64, vp, vp, vp, vp, vp, vp, vp, vp, vp], i32),
         "iga_wq_min_norm_rows": ([i32, i32, i32, vp, vp, vp, C.c_double, vp], i32),
         "iga_wq_point_counts": ([i32, i32, vp, i32, vp, vp, vp], i32),
@@ -254,6 +255,7 @@ def exported_symbols():
         "iga_mft_smem_bytes",
         "iga_mft_matvec",
         "iga_geometry_pointwise",
+        "iga_geometry_coefficients",
         "iga_nurbs_coefficients",
         "iga_wq_min_norm_rows",
         "iga_wq_point_counts",

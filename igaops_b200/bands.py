@@ -253,6 +253,29 @@ class RuleBands:
         return hit
 
 
+def basis_band(q):
+    """Shared band of a rule's B0 and B1, (start, [B0, B1], width, monotone, unit):
+    `unit` tells whether the start advances by at most one per point."""
+    slot = _CACHE.slot(q)
+    hit = slot.get("basisband")
+    if hit is None:
+        start, vals, w, monotone = band_from([q.basis[0], q.basis[1]], unit_steps=True)
+        hit = (start, vals, w, monotone, bool(np.all(np.diff(start) <= 1)))
+        slot["basisband"] = hit
+    return hit
+
+
+def basis_device(q, width: int) -> DeviceBand:
+    """FP64 device form of basis_band padded to `width`."""
+    slot = _CACHE.slot(q)
+    key = ("basisdev", width, torch.cuda.current_device())
+    hit = slot.get(key)
+    if hit is None:
+        hit = _repad(basis_band(q)[:4], width, int(q.nbctrlpts), torch.float64)
+        slot[key] = hit
+    return hit
+
+
 def _same(A, B) -> bool:
     A = sp.csr_array(A)
     B = sp.csr_array(B)

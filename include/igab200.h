@@ -581,6 +581,17 @@ iga_status iga_geometry_pointwise(int ndim, int ncoord, int64_t nq,
                                   double* invjac_out, double* coef_out,
                                   int32_t* status, iga_stream stream);
 
+/* det J (Nq) and C = det J * J^+ J^{+T} ((3, 3, Nq)) of a 3D patch at every
+ * quadrature point in one pass from its control points (3, N), FP64, direction
+ * 1 fastest.  Of the plan, ndim, width (2..6), n, nq, trial and trial_d1 are
+ * read (FP64 bands whose starts never step back nor advance by more than one
+ * per point).  Either output may be NULL; status bits as in
+ * iga_geometry_pointwise.  Replaces the einsum of tests/test_assemble.py:116-123
+ * on EvaluatedSpline (src/igaops/geometry/mixin/template.py:16-130). */
+iga_status iga_geometry_coefficients(const iga_mf_plan* plan, const double* ctrlpts,
+                                     double* det_out, double* coef_out, int32_t* status,
+                                     iga_stream stream);
+
 /* --------------------------------------------------------------------- */
 /* Rational (NURBS) operators                                             */
 /* --------------------------------------------------------------------- */
