@@ -136,6 +136,7 @@ __global__ void __launch_bounds__(32 * kGeoWarps)
   constexpr int CM = 31 + W + 1;  // control range of 32 points (unit steps), even
   __shared__ double s_t[kGeoWarps][2][3][2][CM];  // plane contracted over direction 2
   __shared__ double s_b1[kGeoWarps][2 * W][32];
+  __shared__ __align__(16) double s_b3[kGeoWarps][2][2 * W];  // band values of this and the next point
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int n1 = a.n[0], n2 = a.n[1], n3 = a.n[2];
   const int nq1 = a.nq[0], nq2 = a.nq[1], nq3 = a.nq[2];
@@ -160,9 +161,15 @@ __global__ void __launch_bounds__(32 * kGeoWarps)
   const int64_t plane = (int64_t)n1 * n2, N = plane * n3, Nq = (int64_t)nq1 * nq2 * nq3;
   double F[3][3][W];  // [coordinate][d1, d2, value][plane]
   int buf = 0;
+  // lane l touches a line of the next plane's 3 W rows (two lines cover the usual
+  // 14 control points of 32 points), so that its reads hit L1
+  const int prow = min(lane >> 1, 3 * W - 1);
+  const double* pre = a.x + (prow / W) * N + (int64_t)min(c2lo + prow % W, n2 - 1) * n1 +
+                      min(c1lo + (lane & 1) * (C1r - 1), n1 - 1);
   auto produce = [&](int c3) {
     buf ^= 1;
     const double* xp = a.x + min(c3, n3 - 1) * plane;
+    asm volatile("prefetch.global.L1 [%0];" ::"l"(pre + min(c3 + 1, n3 - 1) * plane));
     for (int e = lane; e < 2 * C1r; e += 32) {
       const int b = e >= C1r, c = e - b * C1r;
       const double* bv = (b ? a.v1[1] : a.v0[1]) + (int64_t)q2 * W;
@@ -206,16 +213,28 @@ __global__ void __launch_bounds__(32 * kGeoWarps)
   int flags = 0;
   double* out = a.coef + ((int64_t)qa * nq2 + q2) * nq1 + q1;
   double* dout = a.det + ((int64_t)qa * nq2 + q2) * nq1 + q1;
+  // the next point's band values travel through a register of lanes 0 .. 2 W - 1
+  auto band3 = [&](int q) {
+    const int k = lane % W;
+    return __ldg((lane < W ? a.v0[2] : a.v1[2]) + (int64_t)min(q, nq3 - 1) * W + k);
+  };
+  double nb = band3(qa);
+  int s3n = __ldg(a.start[2] + qa);
 #pragma unroll 1
   for (int q = qa; q < qb; ++q) {
-    const int s3 = __ldg(a.start[2] + q);
+    double* b3 = s_b3[warp][q & 1];
+    if (lane < 2 * W) b3[lane] = nb;
+    const int s3 = s3n;
+    nb = band3(q + 1);
+    s3n = __ldg(a.start[2] + min(q + 1, nq3 - 1));
     while (base < s3) produce(++base + W - 1);
+    __syncwarp();
     double J[3][3];
 #pragma unroll
     for (int m = 0; m < 3; ++m) J[m][0] = J[m][1] = J[m][2] = 0.0;
 #pragma unroll
     for (int k = 0; k < W; ++k) {
-      const double w0 = __ldg(a.v0[2] + (int64_t)q * W + k), w1 = __ldg(a.v1[2] + (int64_t)q * W + k);
+      const double w0 = b3[k], w1 = b3[W + k];
 #pragma unroll
       for (int m = 0; m < 3; ++m) {
         J[m][0] += w0 * F[m][0][k];
