@@ -4,6 +4,7 @@
 
 #include "mf_fused.cuh"
 #include "mf_warp.cuh"
+#include "mf_warp2.cuh"
 
 namespace iga {
 
@@ -48,19 +49,21 @@ static iga_status check_plan(const iga_mf_plan* p) {
   return IGA_OK;
 }
 
-// The face selects the 3D kernel: 8 x 8 is the warp-per-tile kernel, whose
-// chunks hold the whole tile (padding pencils zero).
+// The face selects the kernel: 8 x 8 (3D) and 32 (2D) are the warp-per-tile
+// kernels, whose chunks hold the whole tile (padding pencils zero).
 static bool warp_face(const iga_mf_plan* p) {
-  return p->ndim == 3 && p->face[0] == kWarpFace && p->face[1] == kWarpFace;
+  return p->ndim == 3 ? p->face[0] == kWarpFace && p->face[1] == kWarpFace
+                      : p->face[0] == kWarpFace2;
 }
 
 static int64_t layout_elems(const iga_mf_plan* p, int dtype, int64_t* tile_off) {
   if (warp_face(p)) {
-    const int64_t tiles = ceil_div(p->nq[0], p->face[0]) * ceil_div(p->nq[1], kWarpFace);
+    const bool d3 = p->ndim == 3;
+    const int64_t tiles = ceil_div(p->nq[0], p->face[0]) * (d3 ? ceil_div(p->nq[1], kWarpFace) : 1);
     // [group][tile][point][stream][pencil]: a tile has no offset of its own
     if (tile_off)
       for (int64_t t = 0; t < tiles; ++t) tile_off[t] = 0;
-    return tiles * p->nq[2] * p->nstream * kWarpTile;
+    return tiles * p->nq[p->ndim - 1] * p->nstream * (d3 ? kWarpTile : kWarpFace2);
   }
   const int FX = p->face[0];
   const int FY = p->ndim == 3 ? p->face[1] : 1;
@@ -137,14 +140,16 @@ __global__ void __launch_bounds__(256) mf_pack3_pm_kernel(int nq1, int nq2, int 
   for (int s = 0; s < S; ++s) dst[s] = (Tout)coefs[(int64_t)rows.r[s] * ld + q];
 }
 
-// pack for the warp-per-tile kernel, [group][tile][point][stream][pencil]: one
-// CTA per (row of tiles, q3); a warp walks one row of points (coalesced reads)
-// and writes its 8-point pieces into the row's tiles, zeros beyond the grid.
-template <typename Tin, typename Tout>
+// pack for the warp-per-tile kernels, [group][tile][point][stream][pencil], tiles
+// of F1 x F2 pencils (F2 = 1 in 2D, where nq2 = 1 and q3 counts direction 2): one
+// CTA per (row of tiles, q3); a warp walks one row of points (coalesced reads) and
+// writes its F1-point pieces into the row's tiles, zeros beyond the grid.
+template <typename Tin, typename Tout, int F1, int F2>
 __global__ void __launch_bounds__(256)
     mf_pack_warp_kernel(int nq1, int nq2, int nq3, int S, int tiles1, int tiles2,
                         const int32_t* __restrict__ groups, SrcRows rows,
                         const Tin* __restrict__ coefs, int64_t ld, Tout* __restrict__ packed) {
+  constexpr int FT = F1 * F2;
   const int t2 = blockIdx.x, q3 = blockIdx.y;
   int lo = 0, hi = __ldg(groups);  // the group of q3
   while (hi - lo > 1) {
@@ -153,16 +158,15 @@ __global__ void __launch_bounds__(256)
     else hi = mid;
   }
   const int qg = __ldg(groups + 1 + lo) >> 2, np = (__ldg(groups + 2 + lo) >> 2) - qg;
-  const int64_t chunk = (int64_t)S * kWarpTile, tstride = np * chunk;
+  const int64_t chunk = (int64_t)S * FT, tstride = np * chunk;
   Tout* base = packed + ((int64_t)qg * tiles1 * tiles2 + (int64_t)t2 * tiles1 * np + (q3 - qg)) * chunk;
-  for (int row = threadIdx.x >> 5; row < S * kWarpFace; row += 8) {
-    const int s = row / kWarpFace, l2 = row % kWarpFace;
-    const int q2 = t2 * kWarpFace + l2;
+  for (int row = threadIdx.x >> 5; row < S * F2; row += 8) {
+    const int s = row / F2, l2 = row % F2;
+    const int q2 = t2 * F2 + l2;
     const Tin* src = coefs + (int64_t)rows.r[s] * ld + ((int64_t)q3 * nq2 + q2) * nq1;
-    Tout* dst = base + s * kWarpTile + l2 * kWarpFace;
-    for (int q1 = threadIdx.x & 31; q1 < tiles1 * kWarpFace; q1 += 32)
-      dst[(q1 / kWarpFace) * tstride + q1 % kWarpFace] =
-          (q1 < nq1 && q2 < nq2) ? (Tout)src[q1] : Tout(0);
+    Tout* dst = base + s * FT + l2 * F1;
+    for (int q1 = threadIdx.x & 31; q1 < tiles1 * F1; q1 += 32)
+      dst[(q1 / F1) * tstride + q1 % F1] = (q1 < nq1 && q2 < nq2) ? (Tout)src[q1] : Tout(0);
   }
 }
 
@@ -238,6 +242,32 @@ static int64_t group_list_bytes(const iga_mf_plan* p, int dtype) {
   const int nq = p->nq[p->ndim - 1];
   return dtype == IGA_F64 ? group_list_offset<double>(nq, n * step_group<double>(p->width))
                           : group_list_offset<float>(nq, n * step_group<float>(p->width));
+}
+
+// resident CTAs of the 2D warp-per-tile kernel: the register budget's, or what
+// shared memory holds (the weight table grows with the test rows' width)
+template <typename T>
+static int warp2_resident(const iga_mf_plan* p) {
+  auto f = [&](auto pat) {
+    using P = decltype(pat);
+    const int kw = std::min(p->rwidth, kWarpFace2);
+    switch (p->width) {
+      case 3: return WarpSmem2<T, P, 3>::total(kw);
+      case 4: return WarpSmem2<T, P, 4>::total(kw);
+      case 5: return WarpSmem2<T, P, 5>::total(kw);
+      default: return WarpSmem2<T, P, 6>::total(kw);
+    }
+  };
+  int smem;
+  switch (p->op) {
+    case IGA_OP_MASS: smem = f(Pat<2, IGA_OP_MASS, 0, 0, 0, 0>{}); break;
+    case IGA_OP_STIFF:
+      smem = p->sym ? f(Pat<2, IGA_OP_STIFF, 0, 0, 0, 1>{}) : f(Pat<2, IGA_OP_STIFF, 0, 0, 0, 0>{});
+      break;
+    case IGA_OP_GRADU_V: smem = f(Pat<2, IGA_OP_GRADU_V, 0, 0, 0, 0>{}); break;
+    default: smem = f(Pat<2, IGA_OP_U_GRADV, 0, 0, 0, 0>{});
+  }
+  return std::min(kWarpResident2, 228 * 1024 / (smem + 1024));
 }
 
 template <typename T>
@@ -544,7 +574,10 @@ iga_status iga_mf_resident(const iga_mf_plan* plan, int dtype, int32_t* ctas) {
   if (rc) return rc;
   IGA_CHECK_ARG(dtype == IGA_F64 || dtype == IGA_F32, "dtype %d not supported", dtype);
   IGA_CHECK_ARG(ctas, "null ctas");
-  *ctas = warp_face(plan) ? warp_resident(dtype == IGA_F64, plan->nstream, plan->width) : 0;
+  *ctas = !warp_face(plan)    ? 0
+          : plan->ndim == 3 ? warp_resident(dtype == IGA_F64, plan->nstream, plan->width)
+          : dtype == IGA_F64  ? warp2_resident<double>(plan)
+                              : warp2_resident<float>(plan);
   return IGA_OK;
 }
 
@@ -615,17 +648,26 @@ iga_status iga_mf_pack(const iga_mf_plan* plan, int dtype_in, const void* coefs,
   for (int d = 0; d < plan->ndim; ++d) Nq *= plan->nq[d];
   IGA_CHECK_ARG(ld >= Nq, "ld %lld smaller than Nq %lld", (long long)ld, (long long)Nq);
   if (warp_face(plan)) {
-    const int nq3 = plan->nq[2], tiles1 = (int)ceil_div(plan->nq[0], plan->face[0]);
+    const bool d3 = plan->ndim == 3;
+    const int nq2 = d3 ? plan->nq[1] : 1, nq3 = plan->nq[plan->ndim - 1];
+    const int tiles1 = (int)ceil_div(plan->nq[0], plan->face[0]);
+    const int tiles2 = d3 ? (int)ceil_div(nq2, kWarpFace) : 1;
     IGA_CHECK_ARG(nq3 <= 65535, "streamed direction of %d points exceeds the grid", nq3);
-    const int tiles2 = (int)ceil_div(plan->nq[1], kWarpFace);
-    IGA_CHECK_ARG(plan->step_table, "face (8, 8) packs by the step table's groups (iga_mf_table)");
+    IGA_CHECK_ARG(plan->step_table, "this face packs by the step table's groups (iga_mf_table)");
     const dim3 grid((unsigned)tiles2, (unsigned)nq3);
     const int32_t* groups =
         (const int32_t*)((const char*)plan->step_table + group_list_bytes(plan, dtype_out));
-#define IGA_PACK(TI, TO)                                                                     \
-  mf_pack_warp_kernel<TI, TO><<<grid, 256, 0, st>>>(plan->nq[0], plan->nq[1], nq3, S, tiles1, \
-                                                    tiles2, groups, rows, (const TI*)coefs,  \
-                                                    ld, (TO*)packed)
+#define IGA_PACK(TI, TO)                                                                         \
+  do {                                                                                           \
+    if (d3)                                                                                      \
+      mf_pack_warp_kernel<TI, TO, kWarpFace, kWarpFace>                                          \
+          <<<grid, 256, 0, st>>>(plan->nq[0], nq2, nq3, S, tiles1, tiles2, groups, rows,         \
+                                 (const TI*)coefs, ld, (TO*)packed);                             \
+    else                                                                                         \
+      mf_pack_warp_kernel<TI, TO, kWarpFace2, 1>                                                 \
+          <<<grid, 256, 0, st>>>(plan->nq[0], nq2, nq3, S, tiles1, tiles2, groups, rows,         \
+                                 (const TI*)coefs, ld, (TO*)packed);                             \
+  } while (0)
     if (dtype_in == IGA_F64 && dtype_out == IGA_F64) IGA_PACK(double, double);
     else if (dtype_in == IGA_F64 && dtype_out == IGA_F32) IGA_PACK(double, float);
     else if (dtype_in == IGA_F32 && dtype_out == IGA_F64) IGA_PACK(float, double);

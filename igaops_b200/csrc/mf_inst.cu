@@ -3,6 +3,7 @@
 // template instances build in parallel.
 #include "mf_fused.cuh"
 #include "mf_warp.cuh"
+#include "mf_warp2.cuh"
 
 #ifndef IGA_INST_D
 #define IGA_INST_D 3
@@ -59,6 +60,22 @@ static iga_status launch_pat(const FusedArgs<T>& a, const LaunchInfo& li) {
     }
     kern<<<grid, FX * FY, smem, li.stream>>>(a);
   } else {
+    if (li.FX == kWarpFace2) {
+      using L = WarpSmem2<T, P, W>;
+      if (!a.step_table) {
+        set_error("2D fused kernel needs the step table of the plan (iga_mf_table)");
+        return IGA_ERR_INVALID_ARG;
+      }
+      if (a.dmax1 > L::nout) {
+        set_error("test range %d of a tile exceeds %d", a.dmax1, L::nout);
+        return IGA_ERR_UNSUPPORTED;
+      }
+      static_assert(L::wtab + 2 * kWarpFace2 * L::nout * (int)sizeof(T) <= 48 * 1024,
+                    "shared memory of a CTA (no opt-in)");
+      mfw2_kernel<T, W, P><<<grid, 32, L::total(std::min(a.RW, kWarpFace2)), li.stream>>>(a);
+      IGA_LAUNCH_CHECK();
+      return IGA_OK;
+    }
     constexpr int FX = kFace2X;
     constexpr int NST = kStages;
     if (li.FX != FX) {

@@ -160,12 +160,13 @@ def _src_rows(ndim, op, st, sym, lead2: int):
     return rows
 
 
-# 3D tiles are 8 x 8, one warp each (csrc/mf_warp.cuh): faster than the 16 x 8
-# CTA-per-tile kernel at every degree, type and size timed (8^3 to 128^3)
+# 3D tiles are 8 x 8, 2D tiles 32 x 1, one warp each (csrc/mf_warp.cuh,
+# mf_warp2.cuh): faster than the CTA-per-tile kernels (faces (16, 8) and (128,)) at
+# every degree, type and size timed (3D 8^3 to 128^3, 2D 8^2 to 320^2)
 FACE3 = (8, 8)
-FACE2 = (128,)
+FACE2 = (32,)
 _SM_COUNT = 148
-_GROUP_POINTS = 3  # points per group of the 3D kernel (kGroupPts)
+_GROUP_POINTS = 3  # points per group of the warp-per-tile kernels (kGroupPts)
 
 
 class FusedPlan:
@@ -208,8 +209,8 @@ class FusedPlan:
         tiles1 = -(-self.nq[0] // face[0])
         tiles2 = -(-self.nq[1] // face[1]) if ndim == 3 else 1
         nlast = self.nq[-1]
-        # 3D: groups of points between window moves, the unit segments are cut in
-        self.groups = rbs[-1].group_count(_GROUP_POINTS) if ndim == 3 else 0
+        # groups of points between window moves, the unit segments are cut in
+        self.groups = rbs[-1].group_count(_GROUP_POINTS)
         self.tiles = tiles1 * tiles2
         P.nseg = 1
         # tile ranges for shared-memory sizing
@@ -234,19 +235,11 @@ class FusedPlan:
             P.testR_d1[d] = testR.vals[1].data_ptr()
         self.status = torch.zeros(1, dtype=torch.int32, device=dev)
         P.status = self.status.data_ptr()
-        self.resident = 0
-        if ndim == 3:
-            res = ctypes.c_int32(0)
-            _lib.check(_lib.LIB.iga_mf_resident(ctypes.byref(P), iga_dtype(dtype),
-                                                ctypes.byref(res)))
-            self.resident = int(res.value)
+        res = ctypes.c_int32(0)
+        _lib.check(_lib.LIB.iga_mf_resident(ctypes.byref(P), iga_dtype(dtype), ctypes.byref(res)))
+        self.resident = int(res.value)
         if nseg is None:
-            if ndim == 3:
-                nseg = self.predicted_nseg()[0]
-            else:
-                # about 12 CTAs per SM, segments of at least 48 points so window
-                # warm-up and flush stay amortised
-                nseg = max(1, min(-(-_SM_COUNT * 12 // self.tiles), nlast // 48))
+            nseg = self.predicted_nseg()[0]
         nseg = max(1, min(int(nseg), nlast))
         P.nseg = nseg
         self.nseg = nseg
@@ -272,7 +265,7 @@ class FusedPlan:
         self.P = P
 
     def predicted_nseg(self, most: int = 64):
-        """Segment counts of the 3D kernel, the one that should run fastest first.
+        """Segment counts, the one that should run fastest first.
 
         Units (tile x segment, one warp each) run in waves of 148 x resident
         warps.  A unit costs its share of the groups plus a fixed part (set-up,

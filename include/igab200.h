@@ -137,8 +137,9 @@ typedef struct {
   int32_t n[3], nq[3];
   int32_t face[2];    /* quadrature tile face (FX, FY): 3D (8, 8), one warp
                          per tile (cmax, dmax <= width + 7), or (16, 8), one
-                         128-thread CTA per tile; 2D (128, 1).  Layout, step
-                         table and packed data belong to a face            */
+                         128-thread CTA per tile; 2D (32, 1), one warp per
+                         tile (dmax <= width + 31), or (128, 1).  Layout,
+                         step table and packed data belong to a face       */
   int32_t nseg;       /* segments of the streamed (last) direction      */
   int32_t nstream;    /* packed coefficient streams                     */
   int32_t src_row[9]; /* leading index of the reference coefficient array
@@ -170,14 +171,14 @@ typedef struct {
 iga_status iga_mf_layout(const iga_mf_plan* plan, int dtype, int64_t* elems,
                          int64_t* tile_off_host);
 
-/* Resident CTAs per SM of the plan's 3D kernel with face (8, 8), for choosing
- * nseg; 0 for the other faces. */
+/* Resident CTAs per SM of the plan's warp-per-tile kernel (faces (8, 8) and
+ * (32, 1)), for choosing nseg; 0 for the other faces. */
 iga_status iga_mf_resident(const iga_mf_plan* plan, int dtype, int32_t* ctas);
 
 /* Step table of the streamed (last) direction: one row per quadrature
  * point holding its trial band values (B0, B1) and test band values (W0^T,
- * W1^T), each padded to 16 bytes; face (8, 8): only the orders the operator
- * reads, then the list of point groups between window moves (iga_mf_pack reads
+ * W1^T), each padded to 16 bytes; faces (8, 8) and (32, 1): only the orders the
+ * operator reads, then the list of point groups between window moves (iga_mf_pack reads
  * it); other faces: all four, then the two band starts.  With table == NULL
  * only *elems is returned; otherwise the rows are written to `table`
  * (caller-owned, *elems elements of `dtype`).  plan->step_table must point
