@@ -174,6 +174,7 @@ def _load():
         "iga_fd_sptime_qz_apply": ([i32, i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, C.c_double,
                                     vp, i32, vp, vp, vp, vp, vp, vp], i32),
         "iga_fd_apply_tc": ([i32, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp, vp], i32),
+        "iga_arnoldi_cgs2": ([i64, i32, vp, i64, vp, i64, vp, vp, i64, vp], i32),
         "iga_gmres_workspace": ([i64, i32, C.POINTER(C.c_int64)], i32),
         "iga_gmres_solve": ([i64, vp, vp, C.c_double, i32, APPLY_FN, APPLY_FN, vp, vp, i64, vp,
                              i64, vp, C.POINTER(C.c_int), vp], i32),
@@ -280,6 +281,7 @@ def exported_symbols():
         "iga_fd_sptime_apply",
         "iga_fd_sptime_qz_apply",
         "iga_fd_apply_tc",
+        "iga_arnoldi_cgs2",
         "iga_gmres_workspace",
         "iga_gmres_solve",
         "iga_gram_workspace",

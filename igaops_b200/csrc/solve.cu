@@ -36,6 +36,33 @@ iga_status iga_axpby(int dtype, int64_t n, double alpha, const void* x, double b
 iga_status iga_mask_zero(int dtype, int64_t nidx, const int64_t* idx, void* x,
                          iga_stream stream);
 
+iga_status iga_arnoldi_cgs2(int64_t n, int it, double* V, int64_t ldv, const double* Z, int64_t ldz,
+                            double* hd, double* partial, int64_t partial_elems,
+                            iga_stream stream) {
+  clear_error();
+  IGA_CHECK_ARG(n >= 1 && it >= 1 && V && hd && partial && ldv >= n && (!Z || ldz >= n),
+                "bad argument");
+  int nblk = 0;
+  int64_t need = 0;
+  iga_status rc = iga_gram_workspace(n, it, 1, 0, &nblk, &need);
+  if (rc) return rc;
+  IGA_CHECK_ARG(partial_elems >= need, "partial buffer holds %lld elements, %lld needed",
+                (long long)partial_elems, (long long)need);
+  double* w = V + (int64_t)it * ldv;
+  for (int pass = 0; pass < 2; ++pass) {
+    double* h = hd + (int64_t)pass * it;
+    if ((rc = iga_gram(IGA_F64, 0, n, it, V, ldv, 1, w, ldv, h, partial, nblk, stream))) return rc;
+    if ((rc = iga_combine(IGA_F64, 0, n, it, V, ldv, 1, h, -1.0, 1.0, w, ldv, stream))) return rc;
+  }
+  if (Z && (rc = iga_gram(IGA_F64, 0, n, it, Z, ldz, 1, Z + (int64_t)(it - 1) * ldz, ldz,
+                          hd + 2 * it, partial, nblk, stream)))
+    return rc;
+  if ((rc = iga_gram_workspace(n, 1, 1, 0, &nblk, &need))) return rc;
+  IGA_CHECK_ARG(partial_elems >= need, "partial buffer holds %lld elements, %lld needed",
+                (long long)partial_elems, (long long)need);
+  return iga_gram(IGA_F64, 0, n, 1, w, ldv, 1, w, ldv, hd + 3 * it, partial, nblk, stream);
+}
+
 iga_status iga_gmres_workspace(int64_t n, int maxiters, int64_t* elems) {
   clear_error();
   IGA_CHECK_ARG(n >= 1 && maxiters >= 1 && maxiters <= 4000 && elems, "bad argument");

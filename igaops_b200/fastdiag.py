@@ -329,12 +329,19 @@ class SpaceFD:
         hit = self._dev.get(dtype)
         if hit is None:
             dev = require_cuda()
-            hit = []
+            hit, args = [], []
             for ii in range(self._nbDoFsPerNode):
                 U = [torch.from_numpy(np.ascontiguousarray(u)).to(dev, dtype)
                      for u in self._eigenvec_by_dir_space[ii]]
                 inv = torch.from_numpy(1.0 / eig[ii]).to(dev, dtype)
                 hit.append((U, inv))
+                # the call's constant arguments
+                lo, mm = self._boxes[ii]
+                arr = ctypes.c_int32 * len(mm)
+                n = arr(*[self._nonzeros_by_dir[d] for d in self._space_dirs])
+                ptrs = (ctypes.c_void_p * len(mm))(*[u.data_ptr() for u in U])
+                args.append((len(mm), n, arr(*lo), arr(*mm), ptrs, math.prod(mm)))
+            self._dev[("args", dtype)] = args
             self._dev[dtype] = hit
         return hit
 
@@ -342,20 +349,17 @@ class SpaceFD:
                      work: Optional[Tuple[torch.Tensor, torch.Tensor]] = None):
         """y = P^{-1} x for one DOF-per-node block; x, y (N*ncols) with the
         column index fastest; device hot path (no host sync)."""
-        U, inv = self.device_data(x.dtype)[node]
-        lo, mm = self._boxes[node]
-        ndim = len(mm)
-        n = [self._nonzeros_by_dir[d] for d in self._space_dirs]
-        M = math.prod(mm)
+        inv = self.device_data(x.dtype)[node][1]
+        ndim, n, lo, mm, ptrs, M = self._dev[("args", x.dtype)][node]
         if work is None:
-            work = (torch.empty(M * ncols, dtype=x.dtype, device=x.device),
-                    torch.empty(M * ncols, dtype=x.dtype, device=x.device))
-        arr = ctypes.c_int32 * ndim
-        ptrs = (ctypes.c_void_p * ndim)(*[u.data_ptr() for u in U])
+            work = torch.empty((2, M * ncols), dtype=x.dtype, device=x.device)
+            w0 = work.data_ptr()
+            w1 = w0 + M * ncols * x.element_size()
+        else:
+            w0, w1 = work[0].data_ptr(), work[1].data_ptr()
         _lib.check(
-            _lib.LIB.iga_fd_apply(iga_dtype(x.dtype), ndim, arr(*n), arr(*lo), arr(*mm), ptrs,
-                                  inv.data_ptr(), ncols, x.data_ptr(), y.data_ptr(),
-                                  work[0].data_ptr(), work[1].data_ptr(), stream_handle())
+            _lib.LIB.iga_fd_apply(iga_dtype(x.dtype), ndim, n, lo, mm, ptrs, inv.data_ptr(), ncols,
+                                  x.data_ptr(), y.data_ptr(), w0, w1, stream_handle())
         )
 
     # ---- tensor-core (BF16) apply, 3D, one DOF per node
@@ -441,8 +445,12 @@ class SpaceFD:
     def apply(self, array_in):
         dtype = compute_dtype(array_in)
         x = to_device(array_in, dtype)
-        tail = tuple(x.shape[1:])
         n1 = self._nbDoFsPerNode
+        if n1 == 1 and x.ndim == 1:
+            y = torch.empty_like(x)
+            self.apply_device(x, y)
+            return like_input(y, array_in)
+        tail = tuple(x.shape[1:])
         n2 = x.shape[0] // n1
         k = math.prod(tail) if tail else 1
         xr = x.reshape(n1, n2 * k)

@@ -25,8 +25,12 @@ class Workspace:
         self.device = device
         self.partial = torch.empty(0, dtype=torch.float64, device=device)
         self.out = torch.empty(0, dtype=torch.float64, device=device)
+        self._known = {}  # (n, m1, m2, cplx) -> blocks, both buffers large enough
 
     def ensure(self, n: int, m1: int, m2: int, cplx: int):
+        known = self._known.get((n, m1, m2, cplx))
+        if known is not None:
+            return known
         nblk = ctypes.c_int(0)
         elems = ctypes.c_int64(0)
         _lib.check(_lib.LIB.iga_gram_workspace(n, m1, m2, cplx, ctypes.byref(nblk),
@@ -37,6 +41,7 @@ class Workspace:
         need = m1 * m2 * (2 if cplx else 1)
         if self.out.numel() < need:
             self.out = torch.empty(max(need, 64), dtype=torch.float64, device=self.device)
+        self._known[(n, m1, m2, cplx)] = nblk.value
         return nblk.value
 
 
@@ -59,6 +64,28 @@ def gram(ws: Workspace, A: torch.Tensor, B: torch.Tensor) -> torch.Tensor:
     if cplx:
         return torch.view_as_complex(out.reshape(m1, m2, 2))
     return out.reshape(m1, m2)
+
+
+def gram_into(ws: Workspace, A: torch.Tensor, B: torch.Tensor, out: torch.Tensor):
+    """out[j1 * m2 + j2] = A_j1 . B_j2 (real; FP64, on the device, no host sync)."""
+    m1, n = (1, A.shape[0]) if A.ndim == 1 else A.shape
+    m2 = 1 if B.ndim == 1 else B.shape[0]
+    nblk = ws.ensure(n, m1, m2, 0)
+    _lib.check(_lib.LIB.iga_gram(iga_dtype(A.dtype), 0, n, m1, A.data_ptr(),
+                                 A.stride(0) if A.ndim == 2 else n, m2, B.data_ptr(),
+                                 B.stride(0) if B.ndim == 2 else n, out.data_ptr(),
+                                 ws.partial.data_ptr(), nblk, stream_handle()))
+
+
+def arnoldi_cgs2(ws: Workspace, V: torch.Tensor, it: int, Z: torch.Tensor, hd: torch.Tensor):
+    """Orthogonalise row `it` of V against the rows before it (two classical
+    Gram-Schmidt passes); hd: both projections, Z[:it] . Z[it - 1], squared norm."""
+    n = V.shape[1]
+    ws.ensure(n, it, 1, 0)
+    ws.ensure(n, 1, 1, 0)
+    _lib.check(_lib.LIB.iga_arnoldi_cgs2(n, it, V.data_ptr(), V.stride(0), Z.data_ptr(),
+                                         Z.stride(0), hd.data_ptr(), ws.partial.data_ptr(),
+                                         ws.partial.numel(), stream_handle()))
 
 
 def gram_host(ws: Workspace, A, B) -> np.ndarray:

@@ -41,20 +41,6 @@ from ._device import iga_dtype, require_cuda, stream_handle, to_device
 __all__ = ["MixedPrecisionFGMRES", "RefinedOutput", "EllipticPatchSolver"]
 
 
-def _gram_into(ws: K.Workspace, A: torch.Tensor, B: torch.Tensor, out: torch.Tensor):
-    """out[j1 * m2 + j2] = A_j1 . B_j2 (FP64, on the device, no host sync)."""
-    if A.ndim == 1:
-        A = A.unsqueeze(0)
-    if B.ndim == 1:
-        B = B.unsqueeze(0)
-    m1, n = A.shape
-    m2 = B.shape[0]
-    nblk = ws.ensure(n, m1, m2, 0)
-    _lib.check(_lib.LIB.iga_gram(iga_dtype(A.dtype), 0, n, m1, A.data_ptr(), A.stride(0), m2,
-                                 B.data_ptr(), B.stride(0), out.data_ptr(), ws.partial.data_ptr(),
-                                 nblk, stream_handle()))
-
-
 def _normalize(x: torch.Tensor, sq: torch.Tensor):
     """x /= sqrt(sq[0]) with sq on the device."""
     _lib.check(_lib.LIB.iga_scale_dev(iga_dtype(x.dtype), 0, x.numel(), x.data_ptr(),
@@ -83,7 +69,7 @@ class _Arnoldi:
         self.ws.ensure(n, m + 1, 1, 0)
 
     def start(self, r: torch.Tensor):
-        _gram_into(self.ws, r, r, self.beta2)
+        K.gram_into(self.ws, r, r, self.beta2)
         K.copy(r, self.V[0])
         _normalize(self.V[0], self.beta2)
 
@@ -92,14 +78,14 @@ class _Arnoldi:
         P_into(V[j], self.Z[j])
         A_into(self.Z[j], w)
         hj = self.H[j, : j + 1]
-        _gram_into(self.ws, V[: j + 1], w, hj)
+        K.gram_into(self.ws, V[: j + 1], w, hj)
         K.combine(V[: j + 1], hj.reshape(j + 1, 1), w, alpha=-1.0, beta=1.0)
         h2 = self.h2[: j + 1]
-        _gram_into(self.ws, V[: j + 1], w, h2)
+        K.gram_into(self.ws, V[: j + 1], w, h2)
         K.combine(V[: j + 1], h2.reshape(j + 1, 1), w, alpha=-1.0, beta=1.0)
         _lib.check(_lib.LIB.iga_axpby(_lib.IGA_F64, j + 1, 1.0, h2.data_ptr(), 1.0, hj.data_ptr(),
                                       stream_handle()))
-        _gram_into(self.ws, w, w, self.H[j, j + 1: j + 2])
+        K.gram_into(self.ws, w, w, self.H[j, j + 1: j + 2])
         _normalize(w, self.H[j, j + 1: j + 2])
 
     def host(self, k: int):
@@ -233,7 +219,7 @@ class MixedPrecisionFGMRES:
 
         r = B["r"]
         K.copy(bd, r)
-        _gram_into(outer.ws, bd, bd, B["nrm"])
+        K.gram_into(outer.ws, bd, bd, B["nrm"])
         b_norm = math.sqrt(max(float(B["nrm"].item()), 0.0))
         if b_norm == 0.0:
             out.success, out.true_residual = True, 0.0
@@ -267,7 +253,7 @@ class MixedPrecisionFGMRES:
             # true residual in FP64
             a64(x, r)
             K.axpby(1.0, bd, -1.0, r)
-            _gram_into(outer.ws, r, r, B["nrm"])
+            K.gram_into(outer.ws, r, r, B["nrm"])
             true_rel = math.sqrt(max(float(B["nrm"].item()), 0.0)) / b_norm
             out.history.append(true_rel)
             if true_rel < self.tolerance:

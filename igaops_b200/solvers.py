@@ -302,6 +302,11 @@ class LinearSolver:
                 K.mask(col, self._mask_dev)
                 x[:, k] = col
 
+    def _masked_into(self, y: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
+        K.copy(y.reshape(out.shape), out)
+        self._mask(out)
+        return out
+
     def solve(self, Afun: Callable, b, Pfun: Optional[Callable] = None, x0=None, **mv_args) -> OutputArgs:
         def identity(x):
             return x
@@ -320,7 +325,10 @@ class LinearSolver:
         dev = require_cuda()
         numpy_in = not isinstance(b, torch.Tensor)
 
-        def matvec(x: torch.Tensor) -> torch.Tensor:
+        # `out`: the product goes there, from an x whose Dirichlet DOFs are zero
+        def matvec(x: torch.Tensor, out=None) -> torch.Tensor:
+            if out is not None:
+                return self._masked_into(_as_vec(Afun(x, **mv_args), x), out)
             self._mask(x)
             y = _as_vec(Afun(x, **mv_args), x)
             if y is x:
@@ -328,7 +336,9 @@ class LinearSolver:
             self._mask(y)
             return y
 
-        def precond(x: torch.Tensor) -> torch.Tensor:
+        def precond(x: torch.Tensor, out=None) -> torch.Tensor:
+            if out is not None:
+                return self._masked_into(_as_vec(Pfun(x), x), out)
             self._mask(x)
             y = _as_vec(Pfun(x), x)
             if y is x:
@@ -364,7 +374,13 @@ class LinearSolver:
     def _GMRES(self, Afun, b: torch.Tensor, Pfun, **kw) -> OutputArgs:
         """Unrestarted GMRES, right preconditioned with the stored Z = P V
         (flexible form), two Gram-Schmidt passes, least squares on the
-        Hessenberg matrix each iteration (linear_solver.py:438-525)."""
+        Hessenberg matrix each iteration (linear_solver.py:438-525).
+
+        One device-to-host read per iteration: the projections of both passes,
+        the new norm and the products Z^T z.  The increment criterion's norms
+        come from the Gram matrix of Z (x = Z y, so |x|^2 = y^T Z^T Z y), so x
+        is formed once, at the end; every vector that enters A or P has zero
+        Dirichlet entries already (masked right-hand side and products)."""
         cm = self.convergence_manager
         ws = K.Workspace(b.device)
         n = b.shape[0]
@@ -376,49 +392,40 @@ class LinearSolver:
             return output
         m = int(cm.parameters["iteration"].reference)
         H = np.zeros((m + 1, m))
+        gram = np.zeros((m, m))  # Z^T Z
         V = torch.empty((m + 1, n), dtype=b.dtype, device=b.device)
         Z = torch.empty((m, n), dtype=b.dtype, device=b.device)
         K.axpby(1.0 / r0, b, 0.0, V[0])
-        w = torch.empty_like(b)
-        xold = torch.empty_like(b)
-        diff = torch.empty_like(b)
+        # per iteration: h of pass 1, h of pass 2, Z^T z, the squared norm
+        hd = torch.empty(3 * m + 1, dtype=torch.float64, device=b.device)
         res = [1.0]
+        yold = np.zeros(0)
         converged = False
         for it in range(1, m + 1):
-            z = Pfun(V[it - 1].clone())
-            K.copy(z, Z[it - 1])
-            K.copy(Afun(Z[it - 1].clone()), w)
-            # both projection passes and the new norm stay on the device
-            # until one transfer (same host arithmetic as reading each)
-            hs = []
-            for _ in range(2):
-                h = K.gram(ws, V[:it], w)[:, 0]
-                K.combine(V[:it], h.reshape(it, 1), w, alpha=-1.0, beta=1.0)
-                hs.append(h)
-            hs.append(K.gram(ws, w, w)[0])
-            hv = torch.cat(hs).cpu().numpy()
+            z = Pfun(V[it - 1].clone(), out=Z[it - 1])
+            w = Afun(z.clone(), out=V[it])
+            K.arnoldi_cgs2(ws, V, it, Z, hd)
+            hv = hd[:3 * it + 1].cpu().numpy()
             _check_finite_host(hv, "the Arnoldi step (operator or preconditioner output)")
-            H[:it, it - 1] += hv[:it]
-            H[:it, it - 1] += hv[it:2 * it]
-            nw = float(np.sqrt(max(float(np.real(hv[2 * it])), 0.0)))
+            H[:it, it - 1] = hv[:it] + hv[it:2 * it]
+            gram[:it, it - 1] = gram[it - 1, :it] = hv[2 * it:3 * it]
+            nw = float(np.sqrt(max(float(hv[3 * it]), 0.0)))
             H[it, it - 1] = nw
             if nw != 0:
-                K.axpby(1.0 / nw, w, 0.0, V[it])
+                K.scale(w, 1.0 / nw)
             else:
                 # breakdown (the Krylov space is invariant): the reference keeps
                 # a zero basis vector and lets the least squares finish
-                V[it].zero_()
+                w.zero_()
             mat = H[: it + 1, :it]
             rhs = np.zeros(it + 1)
             rhs[0] = r0
             y = lstsq(mat, rhs, rcond=None)[0]
-            K.copy(x, xold)
-            K.combine(Z[: len(y)], y.reshape(-1, 1), x)
-            K.copy(x, diff)
-            K.axpby(-1.0, xold, 1.0, diff)
-            nd = torch.cat([K.gram(ws, diff, diff)[0], K.gram(ws, x, x)[0]]).cpu().numpy()
-            incr = (float(np.sqrt(max(float(np.real(nd[0])), 0.0)))
-                    / (float(np.sqrt(max(float(np.real(nd[1])), 0.0))) + Constants.SAFEGUARD))
+            dy = y - np.append(yold, 0.0)
+            g = gram[:it, :it]
+            incr = (float(np.sqrt(max(float(dy @ g @ dy), 0.0)))
+                    / (float(np.sqrt(max(float(y @ g @ y), 0.0))) + Constants.SAFEGUARD))
+            yold = y
             r1 = float(np.linalg.norm(rhs - mat @ y))
             res.append(r1 / r0)
             cm.update(curr_iteration=it, curr_absolute=r1, curr_relative=res[-1],
@@ -426,6 +433,8 @@ class LinearSolver:
             if cm.has_converged():
                 converged = True
                 break
+        if len(yold):
+            K.combine(Z[: len(yold)], yold.reshape(-1, 1), x)
         if not converged:
             output.success = False
             warnings.warn(f"No convergence after {m} iterations.")

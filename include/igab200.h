@@ -253,6 +253,15 @@ iga_status iga_mft_matvec(const iga_mft_plan* plan, const double* packed, int64_
  * error status, which ends the solve with that status. */
 typedef iga_status (*iga_apply_fn)(void* user, const double* x, double* y, iga_stream stream);
 
+/* Vector work of one Arnoldi step after the products, FP64: w = row `it` of V is
+ * orthogonalised against rows 0 .. it - 1 by two classical Gram-Schmidt passes.
+ * hd (device, 3 it + 1) receives the projections of both passes, the products
+ * Z_j . Z_{it-1}, j < it (skipped when Z is NULL), and the squared norm of the new
+ * w.  partial: iga_gram_workspace elements for (n, it, 1) and (n, 1, 1). */
+iga_status iga_arnoldi_cgs2(int64_t n, int it, double* V, int64_t ldv, const double* Z,
+                            int64_t ldz, double* hd, double* partial, int64_t partial_elems,
+                            iga_stream stream);
+
 /* Device workspace (elements of FP64) of iga_gmres_solve for n unknowns and
  * maxiters iterations: (2 maxiters + 3) n plus a few reduction partials. */
 iga_status iga_gmres_workspace(int64_t n, int maxiters, int64_t* elems);
