@@ -56,6 +56,42 @@ inline size_t dense_smem(int mb, int cols, int bn, bool two) {
   return (a + (two ? 2 : 1) * xr * (bn + 4)) * 8;
 }
 
+// ------------------------------------------------- device pieces
+__device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
+  asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};"
+               : "+d"(d[0]), "+d"(d[1])
+               : "d"(a), "d"(b));
+}
+__device__ __forceinline__ void cp8(double* dst, const double* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
+}
+template <typename T>
+__device__ __forceinline__ void stage_elem(double* dst, const T* src) {
+  if constexpr (sizeof(T) == 8) cp8(dst, src);
+  else *dst = (double)__ldg(src);
+}
+
+// acc[i] += A(row block i) X(column block) over K: R row blocks at once. A[r][c]
+// at a[r * sr + c * sc], X[c][n] at b[c * ldx + n] (lane offsets included).
+// (ZERO: from zero.)
+template <int R, bool ZERO>
+__device__ __forceinline__ void block_rows(double (&acc)[R][2], const double* a, int sr8, int sc,
+                                           const double* b, int ldx, int kp) {
+  if (ZERO) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) acc[i][0] = acc[i][1] = 0.0;
+  }
+#pragma unroll 2
+  for (int k = 0; k < kp; k += 4) {
+    const double bv = b[k * ldx];
+    double av[R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) av[i] = a[i * sr8 + k * sc];
+#pragma unroll
+    for (int i = 0; i < R; ++i) dmma(acc[i], av[i], bv);
+  }
+}
+
 template <typename T>
 iga_status launch_dense_mode(const DenseMode<T>& p, bool two, bool dependent, cudaStream_t st);
 

@@ -600,6 +600,10 @@ class SpaceTimeFD:
         tail = tuple(x.shape[1:])
         n1 = self.nbDoFsPerNode
         k = math.prod(tail) if tail else 1
+        if n1 == 1 and k == 1:  # the vector itself is the block
+            y = torch.empty_like(x)
+            self.apply_device(x, y, transpose)
+            return like_input(y, array_in)
         xr = x.reshape(n1, -1, k)
         out = torch.empty_like(xr)
         for ii in range(n1):
