@@ -6,7 +6,7 @@ a B200 mostly idle in that form: every iteration is a handful of short
 kernels and host round trips.  ``PatchBatch`` keeps all patches resident and
 runs each step of the iteration for all of them at once:
 
-* one fused matvec launch per band width over every patch of that width
+* one fused matvec launch over every patch
   (``iga_mf_batch_matvec``; FP64 for the outer iteration, FP32 inside);
 * one set of six tensor-core launches for the fast-diagonalisation apply of
   every patch (``iga_fd_tc_batch_apply``, BF16 products, FP32 accumulation);
@@ -26,6 +26,7 @@ the preconditioner alone for ``inner_iters = 0``).
 from __future__ import annotations
 
 import ctypes
+import math
 from dataclasses import dataclass, field
 from typing import Callable, List, Optional, Sequence
 
@@ -142,6 +143,33 @@ class _BatchArnoldi:
         s.combine(self.Z, k, self.y.data_ptr(), m, 1.0, beta, x)
 
 
+# time of a point group by band width, relative to width 4 (96^3 / 128^3 FP64
+# stiffness products: 8.4, 8.9, 11 and 19 ps per point)
+_GROUP_COST = {3: 0.95, 4: 1.0, 5: 1.25, 6: 2.2}
+
+
+def _joint_nseg(plans) -> List[int]:
+    """Segment counts of patches that share one launch.
+
+    Units of all patches fill the SMs together, so what matters is that they cost
+    about the same and are short against the whole: for a target unit cost L every
+    patch is cut into round(groups * cost / L) segments; the launch takes (sum of
+    unit costs) / (resident units) plus about half of the longest unit, a unit
+    paying five groups for its set-up and its first and last window.  The L with
+    the smallest estimate wins."""
+    resident = 148 * min(p.resident for p in plans)
+    best, cost = None, math.inf
+    for length in (2, 3, 4, 6, 8, 11, 15, 20, 27, 36, 48, 64, 96, 128):
+        ns = [max(1, min(round(p.groups * _GROUP_COST[p.W] / length), p.groups // 2 or 1))
+              for p in plans]
+        units = [(p.groups / k + 5) * _GROUP_COST[p.W] for p, k in zip(plans, ns)]
+        total = sum(p.tiles * k * u for p, k, u in zip(plans, ns, units))
+        est = max(total / resident, max(units)) + 0.5 * max(units)
+        if est < cost:
+            best, cost = ns, est
+    return best
+
+
 @dataclass
 class _Patch:
     rules: list
@@ -152,6 +180,7 @@ class _Patch:
     fd: object
     free: np.ndarray
     dirichlet: np.ndarray
+    fixed_nseg: bool = False  # the caller chose the segment counts
 
 
 class PatchBatch:
@@ -189,7 +218,7 @@ class PatchBatch:
         fd.compute_space_eigendecomposition(rules, np.asarray(table, dtype=bool))
         sp = fd.space_preconditioner
         return _Patch(rules, K64.N, K64.plan.W, K64, K32, fd, sp.free_nodes(0),
-                      sp.dirichlet_nodes(0))
+                      sp.dirichlet_nodes(0), isinstance(nseg, int))
 
     def __init__(self, patches: Sequence, nseg=None):
         dev = require_cuda()
@@ -208,15 +237,21 @@ class PatchBatch:
 
     # -------------------------------------------------------------- tables
     def _matvec_tables(self, dtype):
+        """One multi-patch launch per coefficient symmetry (usually one): the
+        kernel takes each patch's band width from its arguments."""
         dt = iga_dtype(dtype)
         groups = {}
         for i, p in enumerate(self.patches):
-            groups.setdefault(p.W, []).append(i)
+            op = p.K64 if dtype == torch.float64 else p.K32
+            groups.setdefault(op.plan.sym, []).append(i)
         out = []
-        for W, idx in sorted(groups.items()):
+        for _, idx in sorted(groups.items()):
             ops = [self.patches[i].K64 if dtype == torch.float64 else self.patches[i].K32
                    for i in idx]
             plans = (_lib.iga_mf_plan * len(idx))(*[o.plan.P for o in ops])
+            if not any(self.patches[i].fixed_nseg for i in idx):
+                for pl, ns in zip(plans, _joint_nseg([o.plan for o in ops])):
+                    pl.nseg = ns
             packed = (ctypes.c_void_p * len(idx))(*[o.packed.data_ptr() for o in ops])
             offs = (ctypes.c_int64 * len(idx))(*[int(self.seg.offs_host[i]) for i in idx])
             nbytes = ctypes.c_int64(0)
@@ -227,11 +262,14 @@ class PatchBatch:
             smem = ctypes.c_int64(0)
             _lib.check(_lib.LIB.iga_mf_batch_prepare(plans, len(idx), dt, packed, offs, base,
                                                      ctypes.byref(ctas), ctypes.byref(smem)))
+            plan0 = _lib.iga_mf_plan.from_buffer_copy(plans[0])
+            if len({pl.width for pl in plans}) > 1:
+                plan0.width = 0  # the mixed-width kernel
             # the kernel reads the skip flag of its group-local patch index:
             # each group gathers the flags of its patches (global indices)
             gidx = torch.tensor(idx, dtype=torch.int64, device=self.device)
             contiguous = idx == list(range(len(idx)))
-            out.append(dict(plan0=plans[0], plans=plans, n=len(idx), table=table, base=base,
+            out.append(dict(plan0=plan0, plans=plans, n=len(idx), table=table, base=base,
                             ctas=int(ctas.value), smem=int(smem.value), ops=ops, gidx=gidx,
                             identity=contiguous,
                             skipbuf=torch.empty(len(idx), dtype=torch.int32, device=self.device)))
@@ -277,7 +315,7 @@ class PatchBatch:
 
     # ---------------------------------------------------------- operators
     def matvec(self, x: torch.Tensor, y: torch.Tensor, skip: Optional[torch.Tensor] = None):
-        """y = K_p x_p for every patch (one launch per band width), Dirichlet
+        """y = K_p x_p for every patch (one launch), Dirichlet
         rows zeroed; patches with skip[p] >= 0 are left at zero."""
         if self.np == 1:
             # one patch: its own operator's launch (arguments as kernel

@@ -443,10 +443,13 @@ static iga_status batch_prepare(const iga_mf_plan* plans, int npatch, const void
     iga_status rc = check_plan(p);
     if (rc) return rc;
     IGA_CHECK_ARG(p->ndim == 3 && !p->spacetime, "patch %d: multi-patch matvec covers 3D space operators", i);
-    IGA_CHECK_ARG(p->op == p0.op && p->sym == p0.sym && p->width == p0.width &&
+    IGA_CHECK_ARG(p->op == p0.op && p->sym == p0.sym &&
+                      (p->width == p0.width || (warp_face(p) && p->op == IGA_OP_STIFF)) &&
                       p->face[0] == p0.face[0] && p->face[1] == p0.face[1] &&
                       (warp_face(p) || (p->face[0] == kFace3X && p->face[1] == kFace3Y)),
-                  "patch %d: operator, symmetry, band width and face must match patch 0", i);
+                  "patch %d: operator, symmetry, face and (but for stiffness with face (8, 8)) band "
+                  "width must match patch 0",
+                  i);
     const int range = p->width + kWarpFace - 1;
     IGA_CHECK_ARG(!warp_face(p) || std::max({p->cmax[0], p->cmax[1], p->dmax[0], p->dmax[1]}) <= range,
                   "patch %d: control ranges of a tile exceed %d", i, range);
@@ -477,6 +480,7 @@ static iga_status batch_dispatch(const BatchLaunch& b, const T* x, T* y);
 
 template <>
 iga_status batch_dispatch<double>(const BatchLaunch& b, const double* x, double* y) {
+  if (b.W == 0) return launch_mf3_multi(b, x, y);
   switch (b.W) {
     case 3: return launch_mf3_batch_f64_w3(b, x, y);
     case 4: return launch_mf3_batch_f64_w4(b, x, y);
@@ -490,6 +494,7 @@ iga_status batch_dispatch<double>(const BatchLaunch& b, const double* x, double*
 
 template <>
 iga_status batch_dispatch<float>(const BatchLaunch& b, const float* x, float* y) {
+  if (b.W == 0) return launch_mf3_multi(b, x, y);
   switch (b.W) {
     case 3: return launch_mf3_batch_f32_w3(b, x, y);
     case 4: return launch_mf3_batch_f32_w4(b, x, y);
@@ -526,7 +531,8 @@ iga_status iga_mf_batch_prepare(const iga_mf_plan* plans, int npatch, int dtype,
   IGA_CHECK_ARG(plans && npatch >= 1 && packed && offsets && table && total_ctas && smem_bytes,
                 "null argument");
   IGA_CHECK_ARG(((uintptr_t)table & 255) == 0, "table must be 256-byte aligned");
-  IGA_CHECK_ARG(plans[0].width >= 3 && plans[0].width <= 6, "band width %d", plans[0].width);
+  for (int i = 0; i < npatch; ++i)
+    IGA_CHECK_ARG(plans[i].width >= 3 && plans[i].width <= 6, "band width %d", plans[i].width);
   if (dtype == IGA_F64)
     return batch_prepare<double>(plans, npatch, packed, offsets, table, total_ctas, smem_bytes);
   if (dtype == IGA_F32)
@@ -550,6 +556,8 @@ iga_status iga_mf_batch_matvec(const iga_mf_plan* plan0, int dtype, int npatch, 
   b.sym = plan0->sym;
   b.W = plan0->width;
   b.warp = warp_face(plan0);
+  IGA_CHECK_ARG(b.W != 0 || (b.warp && b.op == IGA_OP_STIFF && plan0->nstream > 3),
+                "mixed band widths need the stiffness operator with face (8, 8)");
   b.npatch = npatch;
   b.total_ctas = total_ctas;
   b.smem = (size_t)smem_bytes;

@@ -1355,6 +1355,9 @@ struct BatchLaunch {
   IGA_DECL_BATCH(TN, T, 6)
 IGA_DECL_BATCH_W(f64, double)
 IGA_DECL_BATCH_W(f32, float)
+// any band widths, stiffness, warp-per-tile face (mf_multi.cu)
+iga_status launch_mf3_multi(const BatchLaunch& b, const double* x, double* y);
+iga_status launch_mf3_multi(const BatchLaunch& b, const float* x, float* y);
 #undef IGA_DECL_BATCH_W
 #undef IGA_DECL_BATCH
 

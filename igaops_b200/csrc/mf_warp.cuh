@@ -537,14 +537,14 @@ __global__ void __launch_bounds__(32, warp_resident(sizeof(T) == 8, P::S, W))
   mfw_body<T, W, P>(a, blockIdx.x, blockIdx.y);
 }
 
-// Many patches of one pattern and band width in one launch (see
-// mf3d_batch_kernel): patch p owns CTAs [cta0[p], cta0[p+1]).
-template <typename T, int W, class P>
-__global__ void __launch_bounds__(32, warp_resident(sizeof(T) == 8, P::S, W))
-    mfw_batch_kernel(const FusedArgs<T>* __restrict__ args, const int32_t* __restrict__ cta0,
-                     int npatch, const int64_t* __restrict__ offs, const T* xb, T* yb,
-                     const int32_t* __restrict__ skip) {
-  __shared__ FusedArgs<T> sa;
+// Arguments of the CTA's patch in a multi-patch launch (patch p owns CTAs
+// [cta0[p], cta0[p+1]), its vectors start at offs[p]): the patch, or -1 when it is
+// done (its output stays zero).
+template <typename T>
+__device__ __forceinline__ int mfw_batch_args(const FusedArgs<T>* __restrict__ args,
+                                              const int32_t* __restrict__ cta0, int npatch,
+                                              const int64_t* __restrict__ offs, const T* xb, T* yb,
+                                              const int32_t* __restrict__ skip, FusedArgs<T>& sa) {
   int lo = 0, hi = npatch;
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(32, warp_resident(sizeof(T) == 8, P::S, W))
     else hi = mid;
   }
   const int p = lo;
-  if (skip && __ldg(skip + p) >= 0) return;  // patch done: its output stays zero
+  if (skip && __ldg(skip + p) >= 0) return -1;
   const int* src = reinterpret_cast<const int*>(args + p);
   int* dst = reinterpret_cast<int*>(&sa);
   for (int i = threadIdx.x; i < (int)(sizeof(FusedArgs<T>) / sizeof(int)); i += 32) dst[i] = src[i];
@@ -562,6 +562,18 @@ __global__ void __launch_bounds__(32, warp_resident(sizeof(T) == 8, P::S, W))
     sa.y = yb + offs[p];
   }
   __syncwarp();
+  return p;
+}
+
+// Many patches of one pattern and band width in one launch.
+template <typename T, int W, class P>
+__global__ void __launch_bounds__(32, warp_resident(sizeof(T) == 8, P::S, W))
+    mfw_batch_kernel(const FusedArgs<T>* __restrict__ args, const int32_t* __restrict__ cta0,
+                     int npatch, const int64_t* __restrict__ offs, const T* xb, T* yb,
+                     const int32_t* __restrict__ skip) {
+  __shared__ FusedArgs<T> sa;
+  const int p = mfw_batch_args<T>(args, cta0, npatch, offs, xb, yb, skip, sa);
+  if (p < 0) return;
   mfw_body<T, W, P>(sa, (int)blockIdx.x - __ldg(cta0 + p), 0);
 }
 

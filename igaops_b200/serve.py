@@ -261,9 +261,9 @@ class SolveServer:
         req = a.req
         made = _materialise(req)
         b = to_device(req.rhs, torch.float64, self.dev).reshape(-1).clone()
-        # fixed launch shape: timing every new request shape would add its
-        # tuning to the request latency
-        patch = PatchBatch.make_patch(req.rules, req.coefs, req.table, nseg=2)
+        # launch shape by the wave model: timing every new request shape would
+        # add its tuning to the request latency
+        patch = PatchBatch.make_patch(req.rules, req.coefs, req.table, nseg="heuristic")
         if made:
             req.coefs = None  # computed here, packed now: free them
         K.mask(b, torch.as_tensor(patch.dirichlet, device=self.dev))

@@ -490,8 +490,10 @@ iga_status iga_mf_batch_table_bytes(int dtype, int npatch, int64_t* bytes);
 
 /* Fill the device table (256-byte aligned, synchronous copies) of a
  * multi-patch fused matvec over plans[0..npatch-1] (3D, no time direction,
- * same op, symmetry, band width and face; each with its packed coefficients
- * and step table as for iga_mf_matvec).  Returns the CTA count of the launch
+ * same op, symmetry and face, and the same band width except for stiffness with
+ * face (8, 8); each with its packed coefficients and step table as for
+ * iga_mf_matvec).  With mixed widths, iga_mf_batch_matvec takes plan0 with
+ * width 0.  Returns the CTA count of the launch
  * and its dynamic shared memory. */
 iga_status iga_mf_batch_prepare(const iga_mf_plan* plans, int npatch, int dtype,
                                 const void* const* packed, const int64_t* offsets,
