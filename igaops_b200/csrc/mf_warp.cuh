@@ -298,9 +298,8 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   };
 
   T win[NCOMBO][W][2];  // trial planes at the lane's pencils
-  auto produce = [&]() {
-    cp_async_wait_all();
-    __syncwarp();
+  // q1 contraction of the landed slab, the next one on its way
+  auto produce_q1 = [&]() {
     const T* xr = xr0 + xflip / E;
     xflip = L::xhalf - xflip;
     fetch();
@@ -324,8 +323,9 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
       if (P::b1_needed(0)) a1w[(b1_slot<P>(0) * ROWS + rb) * F] = v0;
       if (P::b1_needed(1)) a1w[(b1_slot<P>(1) * ROWS + rb) * F] = v1;
     }
-    __syncwarp();
-    T nw[NCOMBO][2];
+  };
+  // q2 contraction into the new plane of the window
+  auto produce_q2 = [&](T (&nw)[NCOMBO][2]) {
 #pragma unroll
     for (int b1 = 0; b1 < 2; ++b1) {
       if (!P::b1_needed(b1)) continue;
@@ -347,7 +347,8 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
         nw[combo_slot<P>(c)][1] = v1;
       }
     }
-    asm volatile("" ::: "memory");
+  };
+  auto shift_win = [&](const T (&nw)[NCOMBO][2]) {
 #pragma unroll
     for (int c = 0; c < NCOMBO; ++c)
 #pragma unroll
@@ -356,6 +357,17 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
         for (int m = 0; m < W - 1; ++m) win[c][m][i] = win[c][m + 1][i];
         win[c][W - 1][i] = nw[c][i];
       }
+  };
+
+  auto produce = [&]() {
+    cp_async_wait_all();
+    __syncwarp();
+    produce_q1();
+    __syncwarp();
+    T nw[NCOMBO][2];
+    produce_q2(nw);
+    asm volatile("" ::: "memory");
+    shift_win(nw);
   };
 
   T acc[I][W][2];  // test planes
@@ -393,9 +405,8 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
     if (in && nt * 8 + 2 * tq < D1r) atomicAdd(yr, (T)c0);
     if (in && nt * 8 + 2 * tq + 1 < D1r) atomicAdd(yr + 1, (T)c1);
   };
-  // the oldest test plane is final: contract it over q2, then q1, add into y
-  auto retire = [&]() {
-    __syncwarp();  // the previous plane's fragments are read
+  // the oldest test plane is final: its entries to shared memory ...
+  auto retire_store = [&]() {
 #pragma unroll
     for (int pr = 0; pr < 4; ++pr) {
       if (!P::tpair_needed(pr)) continue;
@@ -409,21 +420,26 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
       *reinterpret_cast<double2*>(dnw + pair_slot<P>(pr) * kWarpTile) =
           make_double2((double)v0, (double)v1);
     }
-    if (yleft > 0) {
-      __syncwarp();
+  };
+  // ... contracted over q2, then q1, added into y: the first block, and the
+  // others where a control range exceeds eight
+  auto flush_first = [&]() {
+    double ks[2][2];
+    flush_q2(0, ks);
+    flush_q1(0, 0, ks);
+    if (D1r > 8) flush_q1(0, 1, ks);
+  };
+  auto flush_second = [&]() {
+    if (D2r > 8) {
       double ks[2][2];
-      flush_q2(0, ks);
-      flush_q1(0, 0, ks);
-      if (D1r > 8) flush_q1(0, 1, ks);
-      if (D2r > 8) {
-        flush_q2(1, ks);
-        flush_q1(1, 0, ks);
-        if (D1r > 8) flush_q1(1, 1, ks);
-      }
+      flush_q2(1, ks);
+      flush_q1(1, 0, ks);
+      if (D1r > 8) flush_q1(1, 1, ks);
     }
+  };
+  auto shift_acc = [&]() {
     --yleft;
     ydst += pstride;
-    asm volatile("" ::: "memory");
 #pragma unroll
     for (int i = 0; i < I; ++i)
 #pragma unroll
@@ -432,6 +448,35 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
         for (int k = 0; k < W - 1; ++k) acc[i][k][c] = acc[i][k + 1][c];
         acc[i][W - 1][c] = T(0);
       }
+  };
+  auto retire = [&]() {
+    __syncwarp();  // the previous plane's fragments are read
+    retire_store();
+    if (yleft > 0) {
+      __syncwarp();
+      flush_first();
+      flush_second();
+    }
+    asm volatile("" ::: "memory");
+    shift_acc();
+  };
+  // both windows move (the usual case): the two chains share their barriers and
+  // fill each other's latencies
+  auto move = [&]() {
+    cp_async_wait_all();
+    __syncwarp();
+    retire_store();
+    produce_q1();
+    __syncwarp();
+    T nw[NCOMBO][2];
+    produce_q2(nw);
+    if (yleft > 0) {
+      flush_first();
+      flush_second();
+    }
+    asm volatile("" ::: "memory");
+    shift_win(nw);
+    shift_acc();
   };
 
   auto point = [&](const T* cs, const T* row) {
@@ -485,8 +530,13 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   for (int g = ga; g < gb; ++g) {
     const int enew = __ldg(glist + 1 + min(g + NB + 2, ngrp));
     if (g > ga) {  // the segment's first windows are in place
-      if (en[0] & 2) retire();
-      if (en[0] & 1) produce();
+      const int mv = en[0] & 3;
+      if (mv == 3) {
+        move();
+      } else {
+        if (mv & 2) retire();
+        if (mv & 1) produce();
+      }
     }
     const int np = (en[1] >> 2) - (en[0] >> 2);
     const bool ok = mbar_wait_bounded_ns(smem_u32(bars) + slot * 8, parity,
