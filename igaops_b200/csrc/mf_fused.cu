@@ -143,7 +143,7 @@ __global__ void __launch_bounds__(256) mf_pack3_pm_kernel(int nq1, int nq2, int 
 // pack for the warp-per-tile kernels, [group][tile][point][stream][pencil], tiles
 // of F1 x F2 pencils (F2 = 1 in 2D, where nq2 = 1 and q3 counts direction 2): one
 // CTA per (row of tiles, q3); a warp walks one row of points (coalesced reads) and
-// writes its F1-point pieces into the row's tiles, zeros beyond the grid.
+// writes its pieces into the row's tiles (pencil l1 F2 + l2), zeros beyond the grid.
 template <typename Tin, typename Tout, int F1, int F2>
 __global__ void __launch_bounds__(256)
     mf_pack_warp_kernel(int nq1, int nq2, int nq3, int S, int tiles1, int tiles2,
@@ -164,9 +164,9 @@ __global__ void __launch_bounds__(256)
     const int s = row / F2, l2 = row % F2;
     const int q2 = t2 * F2 + l2;
     const Tin* src = coefs + (int64_t)rows.r[s] * ld + ((int64_t)q3 * nq2 + q2) * nq1;
-    Tout* dst = base + s * FT + l2 * F1;
+    Tout* dst = base + s * FT + l2;
     for (int q1 = threadIdx.x & 31; q1 < tiles1 * F1; q1 += 32)
-      dst[(q1 / F1) * tstride + q1 % F1] = (q1 < nq1 && q2 < nq2) ? (Tout)src[q1] : Tout(0);
+      dst[(q1 / F1) * tstride + q1 % F1 * F2] = (q1 < nq1 && q2 < nq2) ? (Tout)src[q1] : Tout(0);
   }
 }
 
@@ -401,11 +401,12 @@ static size_t batch_smem(const iga_mf_plan* p, int rlen) {
   auto f = [&](auto pat) -> size_t {
     using P = decltype(pat);
     if (warp_face(p)) {
+      const bool wide = std::max({p->cmax[0], p->cmax[1], p->dmax[0], p->dmax[1]}) > kWarpFace;
       switch (W) {
-        case 3: return WarpSmem<T, P, 3>::total;
-        case 4: return WarpSmem<T, P, 4>::total;
-        case 5: return WarpSmem<T, P, 5>::total;
-        default: return WarpSmem<T, P, 6>::total;
+        case 3: return wide ? WarpSmem<T, P, 3, true>::total : WarpSmem<T, P, 3, false>::total;
+        case 4: return wide ? WarpSmem<T, P, 4, true>::total : WarpSmem<T, P, 4, false>::total;
+        case 5: return wide ? WarpSmem<T, P, 5, true>::total : WarpSmem<T, P, 5, false>::total;
+        default: return wide ? WarpSmem<T, P, 6, true>::total : WarpSmem<T, P, 6, false>::total;
       }
     }
     return mf3d_smem_bytes<T, P>(kFace3X, kFace3Y, W, RW, rlen, p->cmax[0], p->cmax[1],

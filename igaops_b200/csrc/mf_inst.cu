@@ -23,14 +23,17 @@ static iga_status launch_pat(const FusedArgs<T>& a, const LaunchInfo& li) {
         set_error("3D fused kernel needs the step table of the plan (iga_mf_table)");
         return IGA_ERR_INVALID_ARG;
       }
-      using L = WarpSmem<T, P, W>;
-      if (std::max({a.cmax1, a.cmax2, a.dmax1, a.dmax2}) > L::range) {
+      using N = WarpSmem<T, P, W, false>;
+      using L = WarpSmem<T, P, W, true>;
+      const int range = std::max({a.cmax1, a.cmax2, a.dmax1, a.dmax2});
+      if (range > L::range) {
         set_error("control ranges %d/%d/%d/%d of a tile exceed %d", a.cmax1, a.cmax2, a.dmax1,
                   a.dmax2, L::range);
         return IGA_ERR_UNSUPPORTED;
       }
       static_assert(L::total <= 48 * 1024, "shared memory of a CTA (no opt-in)");
-      mfw_kernel<T, W, P><<<grid, 32, L::total, li.stream>>>(a);
+      if (range > kWarpFace) mfw_kernel<T, W, P, true><<<grid, 32, L::total, li.stream>>>(a);
+      else mfw_kernel<T, W, P, false><<<grid, 32, N::total, li.stream>>>(a);
       IGA_LAUNCH_CHECK();
       return IGA_OK;
     }
@@ -135,8 +138,13 @@ static iga_status launch_pat_batch(const BatchLaunch& b, const T* x, T* y) {
     return IGA_ERR_UNSUPPORTED;
   }
   if (b.warp) {
-    mfw_batch_kernel<T, W, P><<<(unsigned)b.total_ctas, 32, b.smem, b.stream>>>(
-        (const FusedArgs<T>*)b.args, b.cta0, b.npatch, b.offs, x, y, b.skip);
+    // (the wide form's layout is the larger: it tells the two apart)
+    if (b.smem == (size_t)WarpSmem<T, P, W, true>::total)
+      mfw_batch_kernel<T, W, P, true><<<(unsigned)b.total_ctas, 32, b.smem, b.stream>>>(
+          (const FusedArgs<T>*)b.args, b.cta0, b.npatch, b.offs, x, y, b.skip);
+    else
+      mfw_batch_kernel<T, W, P, false><<<(unsigned)b.total_ctas, 32, b.smem, b.stream>>>(
+          (const FusedArgs<T>*)b.args, b.cta0, b.npatch, b.offs, x, y, b.skip);
     IGA_LAUNCH_CHECK();
     return IGA_OK;
   }

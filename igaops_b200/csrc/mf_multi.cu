@@ -16,11 +16,16 @@ __global__ void __launch_bounds__(32, warp_resident(sizeof(T) == 8, P::S, 6))
   const int p = mfw_batch_args<T>(args, cta0, npatch, offs, xb, yb, skip, sa);
   if (p < 0) return;
   const int unit = (int)blockIdx.x - __ldg(cta0 + p);
-  switch (__ldg(&args[p].W)) {
-    case 3: mfw_body<T, 3, P>(sa, unit, 0); break;
-    case 4: mfw_body<T, 4, P>(sa, unit, 0); break;
-    case 5: mfw_body<T, 5, P>(sa, unit, 0); break;
-    default: mfw_body<T, 6, P>(sa, unit, 0);
+  const bool wide = max(max(sa.cmax1, sa.cmax2), max(sa.dmax1, sa.dmax2)) > kWarpFace;
+  switch (2 * sa.W + wide) {
+    case 6: mfw_body<T, 3, P, false>(sa, unit, 0); break;
+    case 7: mfw_body<T, 3, P, true>(sa, unit, 0); break;
+    case 8: mfw_body<T, 4, P, false>(sa, unit, 0); break;
+    case 9: mfw_body<T, 4, P, true>(sa, unit, 0); break;
+    case 10: mfw_body<T, 5, P, false>(sa, unit, 0); break;
+    case 11: mfw_body<T, 5, P, true>(sa, unit, 0); break;
+    case 12: mfw_body<T, 6, P, false>(sa, unit, 0); break;
+    default: mfw_body<T, 6, P, true>(sa, unit, 0);
   }
 }
 

@@ -84,6 +84,20 @@ __host__ __device__ constexpr int a2_slot(int b) {
   return (b == 1 && a2_needed<P>(0)) ? 1 : 0;
 }
 
+// derivative orders of the trial factors of direction 2
+template <class P>
+__host__ __device__ constexpr bool b2_needed(int b) {
+  return P::combo_needed(2 * b) || P::combo_needed(2 * b + 1);
+}
+template <class P>
+__host__ __device__ constexpr int nb2() {
+  return (b2_needed<P>(0) ? 1 : 0) + (b2_needed<P>(1) ? 1 : 0);
+}
+template <class P>
+__host__ __device__ constexpr int b2_slot(int b) {
+  return (b == 1 && b2_needed<P>(0)) ? 1 : 0;
+}
+
 // Points per group: the elements of a type-2 rule have three.
 constexpr int kGroupPts = 3;
 
@@ -100,30 +114,29 @@ __host__ __device__ constexpr int warp_resident(bool f64, int S, int W) {
 }
 
 // Shared memory of a CTA (byte offsets; every region 16-byte aligned). Band
-// starts advance by at most one control plane per point, so a block's control
-// ranges are at most W + 7 wide and every offset is a compile-time constant.
-template <typename T, class P, int W>
+// starts advance by at most one control plane per point, so a tile's control
+// ranges are at most W + 7 wide. WIDE: some tile's range exceeds eight (degree 5,
+// or elements of fewer than three points) and takes a second 8-block.
+template <typename T, class P, int W, bool WIDE>
 struct WarpSmem {
   static constexpr int E = (int)sizeof(T);
-  static constexpr int range = W + kWarpFace - 1;
-  static constexpr int rows = (range + 3) / 4 * 4;          // rows of the slab (whole passes)
-  static constexpr int xrow = range;                        // slab row stride
-  static constexpr int nblk = (range + 7) / 8;              // 8-blocks of a control range
+  static constexpr int range = W + kWarpFace - 1;           // widest control range
+  static constexpr int NBK = WIDE ? 2 : 1;                  // 8-blocks of a range
+  static constexpr int KC = WIDE ? (range + 3) / 4 : 2;     // k-steps over a slab row
+  static constexpr int rows = 8 * NBK;                      // slab rows
+  static constexpr int xrow = KC <= 3 ? 12 : 20;            // slab row stride, 4 mod 8
   static constexpr int row = warp_row_len<T, P>(W);
   static constexpr int chunk = P::S * kWarpTile;            // elements per point
   static constexpr int slot = kGroupPts * (chunk + row);    // elements per group
-  static constexpr int bw = W % 2 ? 2 * W : 2 * W + 2;      // band row stride (conflict-free)
-  __host__ __device__ static constexpr int up(int b) { return (b + 15) / 16 * 16; }
   static constexpr int ring = 64;  // after the mbarriers
-  static constexpr int done = ring + kWarpRing * slot * E;
-  static constexpr int a1s = done + npair3<P>() * kWarpTile * 8;
-  static constexpr int xs = a1s + up(nb1<P>() * rows * kWarpFace * E);
-  static constexpr int xhalf = up(rows * xrow * E);
-  static constexpr int b1 = xs + 2 * xhalf;
-  static constexpr int b2 = b1 + up(kWarpFace * bw * E);
-  static constexpr int f2 = b2 + up(kWarpFace * bw * E);    // [mt][b][kt][lane]
-  static constexpr int f1 = f2 + nblk * na2<P>() * 2 * 32 * 8;  // [nt][g][kt][lane]
-  static constexpr int total = f1 + nblk * ng<P>() * 2 * 32 * 8;
+  static constexpr int xs = ring + kWarpRing * slot * E;
+  static constexpr int xhalf = rows * xrow * E;
+  // weight fragments, 32 doubles each
+  static constexpr int a1 = xs + 2 * xhalf;                 // [b1][kt]: trial bands of q1
+  static constexpr int b2 = a1 + nb1<P>() * KC * 256;       // [b2][block][i]: of q2
+  static constexpr int w2 = b2 + nb2<P>() * NBK * 2 * 256;  // [a2][block][i]: test weights of q2
+  static constexpr int w1 = w2 + na2<P>() * NBK * 2 * 256;  // [a1][block][j]: of q1
+  static constexpr int total = w1 + ng<P>() * NBK * 2 * 256;
 };
 
 // Asynchronous copy of one element to shared memory.
@@ -141,16 +154,15 @@ __host__ __device__ inline int64_t group_list_offset(int nq, int row) {  // byte
   return ((int64_t)nq * row * (int)sizeof(T) + 15) / 16 * 16;
 }
 
-template <typename T, int W, class P>
+template <typename T, int W, class P, bool WIDE>
 __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, const int col) {
-  using L = WarpSmem<T, P, W>;
+  using L = WarpSmem<T, P, W, WIDE>;
   constexpr int S = P::S, I = P::I, J = P::J;
   constexpr int NCOMBO = ncombo3<P>();
   constexpr int NB = kWarpRing;
   constexpr int G = step_group<T>(W);
-  constexpr int F = kWarpFace, XR = L::xrow, ROWS = L::rows, E = L::E;
+  constexpr int F = kWarpFace, XR = L::xrow, E = L::E, NBK = L::NBK;
   static_assert(NB * 8 <= L::ring, "barrier area");
-  static_assert(L::nblk == 2, "two 8-blocks cover a control range");
   extern __shared__ __align__(128) unsigned char smem[];
 
   const int lane = threadIdx.x;
@@ -163,13 +175,7 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
 
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
   T* ring = reinterpret_cast<T*>(smem + L::ring);
-  double* done = reinterpret_cast<double*>(smem + L::done);
-  T* a1s = reinterpret_cast<T*>(smem + L::a1s);
   T* xs = reinterpret_cast<T*>(smem + L::xs);
-  T* b1t = reinterpret_cast<T*>(smem + L::b1);
-  T* b2t = reinterpret_cast<T*>(smem + L::b2);
-  double* f2 = reinterpret_cast<double*>(smem + L::f2);
-  double* f1 = reinterpret_cast<double*>(smem + L::f1);
 
   // ----------------------------------------------------- groups of the segment
   const int* glist = reinterpret_cast<const int*>(reinterpret_cast<const char*>(a.step_table) +
@@ -221,76 +227,92 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   const int D1r = min(__ldg(a.wtstart[0] + q1lo + w1 - 1) + W - 1, n1 - 1) - d1lo + 1;
   const int d2lo = __ldg(a.wtstart[1] + q2lo);
   const int D2r = min(__ldg(a.wtstart[1] + q2lo + w2 - 1) + W - 1, n2 - 1) - d2lo + 1;
-  for (int e = lane; e < F * 2 * W; e += 32) {
-    const int l = e / (2 * W), r = e - l * 2 * W, b = r / W, k = r - b * W;
-    b1t[l * L::bw + r] =
-        __ldg((b ? a.tB1[0] : a.tB0[0]) + (int64_t)(q1lo + min(l, w1 - 1)) * W + k);
-    b2t[l * L::bw + r] =
-        __ldg((b ? a.tB1[1] : a.tB0[1]) + (int64_t)(q2lo + min(l, w2 - 1)) * W + k);
-  }
-  const int gq = lane >> 2, tq = lane & 3;  // fragment coordinates
-  // fragments of the test weights, zero outside the band and the tile.
-  // q2: A operand, rows r2, columns l2 = 4 kt + tq; q1: B operand, rows
-  // l1 = 2 tq + kt, columns r1
+  // Weight fragments (lane = 4 gq + tq holds A[gq][tq] or B[tq][gq]), zero outside
+  // the bands and the tile. A lane's pencils are (q1 = gq, q2 = 2 tq + i), so with
+  // the k index of a product standing for point 2 tq + i (i = k-step) or control
+  // row 2 tq + i, the accumulators of one product are operands of the next.
+  const int gq = lane >> 2, tq = lane & 3;
+  double* fa1 = reinterpret_cast<double*>(smem + L::a1) + lane;
+  double* fb2 = reinterpret_cast<double*>(smem + L::b2) + lane;
+  double* fw2 = reinterpret_cast<double*>(smem + L::w2) + lane;
+  double* fw1 = reinterpret_cast<double*>(smem + L::w1) + lane;
+  {
+    const int q1 = q1lo + min(gq, w1 - 1), q2 = q2lo + min(gq, w2 - 1);
+    const int s1 = __ldg(a.tstart[0] + q1) - c1lo, s2 = __ldg(a.tstart[1] + q2) - c2lo;
+    auto band = [&](const T* v, int q, int k) {
+      return k >= 0 && k < W ? (double)__ldg(v + (int64_t)q * W + k) : 0.0;
+    };
+#pragma unroll
+    for (int b = 0; b < 2; ++b) {
+      if (P::b1_needed(b)) {
+#pragma unroll
+        for (int kt = 0; kt < L::KC; ++kt)
+          fa1[(b1_slot<P>(b) * L::KC + kt) * 32] = band(b ? a.tB1[0] : a.tB0[0], q1, 4 * kt + tq - s1);
+      }
+      if (b2_needed<P>(b)) {
+#pragma unroll
+        for (int m = 0; m < 2 * NBK; ++m)
+          fb2[(b2_slot<P>(b) * 2 * NBK + m) * 32] =
+              band(b ? a.tB1[1] : a.tB0[1], q2, 8 * (m >> 1) + 2 * tq + (m & 1) - s2);
+      }
+    }
 #pragma unroll 1
-  for (int m = 0; m < L::nblk * 4; ++m) {
-    const int r = (m >> 2) * 8 + gq, b = (m >> 1) & 1, kt = m & 1;
-    double v2 = 0.0, v1 = 0.0;
-    if (r < D2r && 4 * kt + tq < w2) {
-      const int k = q2lo + 4 * kt + tq - __ldg(a.rstart[1] + d2lo + r);
-      if (k >= 0 && k < a.RW)
-        v2 = (double)__ldg((b ? a.wR1[1] : a.wR0[1]) + (int64_t)(d2lo + r) * a.RW + k);
+    for (int m = 0; m < 2 * NBK; ++m) {
+      const int r = 8 * (m >> 1) + gq, l = 2 * tq + (m & 1);
+      double v2[2] = {0.0, 0.0}, v1[2] = {0.0, 0.0};
+      if (r < D2r && l < w2) {
+        const int k = q2lo + l - __ldg(a.rstart[1] + d2lo + r);
+        if (k >= 0 && k < a.RW) {
+          const int64_t at = (int64_t)(d2lo + r) * a.RW + k;
+          if (a2_needed<P>(0)) v2[0] = (double)__ldg(a.wR0[1] + at);
+          if (a2_needed<P>(1)) v2[1] = (double)__ldg(a.wR1[1] + at);
+        }
+      }
+      if (r < D1r && l < w1) {
+        const int k = q1lo + l - __ldg(a.rstart[0] + d1lo + r);
+        if (k >= 0 && k < a.RW) {
+          const int64_t at = (int64_t)(d1lo + r) * a.RW + k;
+          if (P::a1_needed(0)) v1[0] = (double)__ldg(a.wR0[0] + at);
+          if (P::a1_needed(1)) v1[1] = (double)__ldg(a.wR1[0] + at);
+        }
+      }
+#pragma unroll
+      for (int b = 0; b < 2; ++b) {
+        if (a2_needed<P>(b)) fw2[(a2_slot<P>(b) * 2 * NBK + m) * 32] = v2[b];
+        if (P::a1_needed(b)) fw1[(g_slot<P>(b) * 2 * NBK + m) * 32] = v1[b];
+      }
     }
-    if (r < D1r && 2 * tq + kt < w1) {
-      const int k = q1lo + 2 * tq + kt - __ldg(a.rstart[0] + d1lo + r);
-      if (k >= 0 && k < a.RW)
-        v1 = (double)__ldg((b ? a.wR1[0] : a.wR0[0]) + (int64_t)(d1lo + r) * a.RW + k);
-    }
-    const int mt = m >> 2;
-    if (b ? a2_needed<P>(1) : a2_needed<P>(0))
-      f2[((mt * na2<P>() + (b ? a2_slot<P>(1) : 0)) * 2 + kt) * 32 + lane] = v2;
-    if (b ? P::a1_needed(1) : P::a1_needed(0))
-      f1[((mt * ng<P>() + (b ? g_slot<P>(1) : 0)) * 2 + kt) * 32 + lane] = v1;
   }
 
   const int64_t pstride = (int64_t)n1 * n2;  // control points per plane
-  // lane roles: production over q1 (column lx, rows r0 + 4 i), production over
-  // q2 and the points (row ly, pencils px, px + 1)
-  const int ly = lane >> 2, px = 2 * (lane & 3);
-  const int lx = lane & 7, r0 = lane >> 3;
-  const int s1 = __ldg(a.tstart[0] + q1lo + min(lx, w1 - 1)) - c1lo;
-  const int s2 = __ldg(a.tstart[1] + q2lo + min(ly, w2 - 1)) - c2lo;
-  const T* b1l = b1t + lx * L::bw;
-  const T* b2l = b2t + ly * L::bw;
-  const T* xr0 = xs + r0 * XR + s1;
-  T* a1w = a1s + r0 * F + lx;
-  const T* a1r = a1s + s2 * F + px;
-  double* dnw = done + ly * F + (px ^ ((ly & 2) << 1));
-  const double* dnr = done + tq * F + (gq ^ ((tq & 2) << 1));
-
   // x slab of one control plane, copied one plane ahead into the other half of
-  // xs: 4 rows x 8 columns per pass, columns beyond the eighth in a remainder
-  // loop. Control points beyond the patch only meet zero band values: their
-  // copies read the nearest point of the patch instead.
-  auto xoff = [&](int r, int c) { return min(r, n2 - 1 - c2lo) * n1 + min(c, n1 - 1 - c1lo); };
-  const int xg0 = xoff(r0, min(lx, C1r - 1)), xg1 = xoff(min(r0 + 4, C2r - 1), min(lx, C1r - 1));
+  // xs, 4 rows x 8 columns per pass (rows paired so that a half-warp's two rows
+  // fall on different banks). Rows and columns past the control range repeat its
+  // last, control points beyond the patch the patch's last: all meet zero weights.
+  const int xr0 = ((lane >> 3) & 1) * 2 + (lane >> 4), xc0 = lane & 7;
+  auto xoff = [&](int r, int c) {
+    return min(min(r, C2r - 1), n2 - 1 - c2lo) * n1 + min(min(c, C1r - 1), n1 - 1 - c1lo);
+  };
+  const int xg0 = xoff(xr0, xc0), xg1 = xoff(xr0 + 4, xc0);
   const T* xsrc = a.x + (int64_t)col * a.N + (int64_t)c2lo * n1 + c1lo;
   int xplane = __ldg(a.tstart[2] + qa);
   xsrc += min(xplane, n3 - 1) * pstride;
-  const uint32_t xdst = smem_u32(xs) + (r0 * XR + lx) * E;
-  const bool wide = C1r > 8 || C2r > 8;
+  const uint32_t xdst = smem_u32(xs) + (xr0 * XR + xc0) * E;
   int xflip = 0;  // half (bytes) that the next copy fills
   auto fetch = [&]() {
     cp_async_elem<E>(xdst + xflip, xsrc + xg0);
     cp_async_elem<E>(xdst + xflip + 4 * XR * E, xsrc + xg1);
-    if (wide) {
-      if (C2r > 8)
-        cp_async_elem<E>(xdst + xflip + 8 * XR * E,
-                         xsrc + xoff(min(r0 + 8, C2r - 1), min(lx, C1r - 1)));
+    if constexpr (WIDE) {
+      if (C2r > 8) {
+        cp_async_elem<E>(xdst + xflip + 8 * XR * E, xsrc + xoff(xr0 + 8, xc0));
+        cp_async_elem<E>(xdst + xflip + 12 * XR * E, xsrc + xoff(xr0 + 12, xc0));
+      }
+      if (C1r > 8) {
+        constexpr int C = 4 * L::KC - 8;  // columns 8 .. 4 KC - 1
 #pragma unroll 1
-      for (int e = lane; e < (C1r - 8) * ROWS; e += 32) {
-        const int c = 8 + e / ROWS, r = e % ROWS;
-        cp_async_elem<E>(smem_u32(xs) + xflip + (r * XR + c) * E, xsrc + xoff(min(r, C2r - 1), c));
+        for (int e = lane; e < C * L::rows; e += 32)
+          cp_async_elem<E>(smem_u32(xs) + xflip + (e / C * XR + 8 + e % C) * E,
+                           xsrc + xoff(e / C, 8 + e % C));
       }
     }
     cp_async_commit();
@@ -298,76 +320,46 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   };
 
   T win[NCOMBO][W][2];  // trial planes at the lane's pencils
-  // q1 contraction of the landed slab, the next one on its way
-  auto produce_q1 = [&]() {
-    const T* xr = xr0 + xflip / E;
+  const T* xl = xs + gq * XR + tq;
+  // the landed slab contracted over q1, then q2 (both on the tensor cores, the
+  // first product's accumulators are the second's A operand); next slab under way
+  auto produce = [&]() {
+    cp_async_wait_all();
+    __syncwarp();
+    const T* xb = xl + xflip / E;
     xflip = L::xhalf - xflip;
+    double d2[NCOMBO][2];
+#pragma unroll
+    for (int c = 0; c < NCOMBO; ++c) d2[c][0] = d2[c][1] = 0.0;
+#pragma unroll
+    for (int nb = 0; nb < NBK; ++nb) {
+      if (nb == 1 && C2r <= 8) break;
+      double d1[2][2];
+      d1[0][0] = d1[0][1] = d1[1][0] = d1[1][1] = 0.0;
+#pragma unroll
+      for (int kt = 0; kt < L::KC; ++kt) {
+        if (kt >= 2 && C1r <= 4 * kt) break;
+        const double xv = (double)xb[8 * nb * XR + 4 * kt];
+        if (P::b1_needed(0)) dmma_8x8x4(d1[0][0], d1[0][1], fa1[kt * 32], xv);
+        if (P::b1_needed(1)) dmma_8x8x4(d1[1][0], d1[1][1], fa1[(b1_slot<P>(1) * L::KC + kt) * 32], xv);
+      }
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (P::combo_needed(c))
+            dmma_8x8x4(d2[combo_slot<P>(c)][0], d2[combo_slot<P>(c)][1], d1[c & 1][i],
+                       fb2[(b2_slot<P>(c >> 1) * 2 * NBK + 2 * nb + i) * 32]);
+    }
     fetch();
-    T bv[2][W];
-#pragma unroll
-    for (int b = 0; b < 2; ++b)
-#pragma unroll
-      for (int k = 0; k < W; ++k)
-        if (P::b1_needed(b)) bv[b][k] = b1l[b * W + k];
-    // rows past the control range hold stale slab entries; nothing reads them
-#pragma unroll
-    for (int rb = 0; rb < ROWS; rb += 4) {
-      if (rb >= 8 && rb >= C2r) break;
-      T v0 = T(0), v1 = T(0);
-#pragma unroll
-      for (int k = 0; k < W; ++k) {
-        const T xv = xr[rb * XR + k];
-        if (P::b1_needed(0)) v0 += bv[0][k] * xv;
-        if (P::b1_needed(1)) v1 += bv[1][k] * xv;
-      }
-      if (P::b1_needed(0)) a1w[(b1_slot<P>(0) * ROWS + rb) * F] = v0;
-      if (P::b1_needed(1)) a1w[(b1_slot<P>(1) * ROWS + rb) * F] = v1;
-    }
-  };
-  // q2 contraction into the new plane of the window
-  auto produce_q2 = [&](T (&nw)[NCOMBO][2]) {
-#pragma unroll
-    for (int b1 = 0; b1 < 2; ++b1) {
-      if (!P::b1_needed(b1)) continue;
-      T xw[W][2];
-#pragma unroll
-      for (int k = 0; k < W; ++k) ld2(a1r + (b1_slot<P>(b1) * ROWS + k) * F, xw[k][0], xw[k][1]);
-#pragma unroll
-      for (int b2 = 0; b2 < 2; ++b2) {
-        const int c = b1 | (b2 << 1);
-        if (!P::combo_needed(c)) continue;
-        T v0 = T(0), v1 = T(0);
-#pragma unroll
-        for (int k = 0; k < W; ++k) {
-          const T bb = b2l[b2 * W + k];
-          v0 += bb * xw[k][0];
-          v1 += bb * xw[k][1];
-        }
-        nw[combo_slot<P>(c)][0] = v0;
-        nw[combo_slot<P>(c)][1] = v1;
-      }
-    }
-  };
-  auto shift_win = [&](const T (&nw)[NCOMBO][2]) {
 #pragma unroll
     for (int c = 0; c < NCOMBO; ++c)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
 #pragma unroll
         for (int m = 0; m < W - 1; ++m) win[c][m][i] = win[c][m + 1][i];
-        win[c][W - 1][i] = nw[c][i];
+        win[c][W - 1][i] = (T)d2[c][i];
       }
-  };
-
-  auto produce = [&]() {
-    cp_async_wait_all();
-    __syncwarp();
-    produce_q1();
-    __syncwarp();
-    T nw[NCOMBO][2];
-    produce_q2(nw);
-    asm volatile("" ::: "memory");
-    shift_win(nw);
   };
 
   T acc[I][W][2];  // test planes
@@ -378,66 +370,54 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   int yleft = n3 - __ldg(a.wtstart[2] + qa);  // planes of y from the oldest one on
   T* ydst = a.y + (int64_t)col * a.N + (int64_t)d2lo * n1 + d1lo + (n3 - yleft) * pstride;
   const int ylane = gq * n1 + 2 * tq;
-  // one 8-row block of the q2 contraction
-  auto flush_q2 = [&](int mt, double (&ks)[2][2]) {
-    ks[0][0] = ks[0][1] = ks[1][0] = ks[1][1] = 0.0;
+  // the oldest test plane is final: contracted over q2 (the accumulators are the B
+  // operand), then q1, and added into y
+  auto retire = [&]() {
+    if (yleft > 0) {
+      double v[4][2];
 #pragma unroll
-    for (int pr = 0; pr < 4; ++pr) {
-      if (!P::tpair_needed(pr)) continue;
+      for (int pr = 0; pr < 4; ++pr) {
+        if (!P::tpair_needed(pr)) continue;
+        T v0 = T(0), v1 = T(0);
 #pragma unroll
-      for (int kt = 0; kt < 2; ++kt)
-        dmma_8x8x4(ks[pr & 1][0], ks[pr & 1][1], f2[((mt * na2<P>() + a2_slot<P>(pr >> 1)) * 2 + kt) * 32 + lane],
-                   dnr[pair_slot<P>(pr) * kWarpTile + kt * 4 * F]);
-    }
-  };
-  // one 8-column block of the q1 contraction of a q2 block
-  auto flush_q1 = [&](int mt, int nt, const double (&ks)[2][2]) {
-    double c0 = 0.0, c1 = 0.0;
+        for (int i = 0; i < I; ++i)
+          if (P::tpair(i) == pr) {
+            v0 += acc[i][0][0];
+            v1 += acc[i][0][1];
+          }
+        v[pr][0] = (double)v0;
+        v[pr][1] = (double)v1;
+      }
 #pragma unroll
-    for (int g = 0; g < 2; ++g) {
-      if (!P::a1_needed(g)) continue;
+      for (int mt = 0; mt < NBK; ++mt) {
+        if (mt == 1 && D2r <= 8) break;
+        double e[2][2];
+        e[0][0] = e[0][1] = e[1][0] = e[1][1] = 0.0;
 #pragma unroll
-      for (int kt = 0; kt < 2; ++kt)
-        dmma_8x8x4(c0, c1, ks[g][kt], f1[((nt * ng<P>() + g_slot<P>(g)) * 2 + kt) * 32 + lane]);
-    }
-    T* yr = ydst + ylane + mt * 8 * n1 + nt * 8;
-    const bool in = mt * 8 + gq < D2r;
-    if (in && nt * 8 + 2 * tq < D1r) atomicAdd(yr, (T)c0);
-    if (in && nt * 8 + 2 * tq + 1 < D1r) atomicAdd(yr + 1, (T)c1);
-  };
-  // the oldest test plane is final: its entries to shared memory ...
-  auto retire_store = [&]() {
+        for (int i = 0; i < 2; ++i)
 #pragma unroll
-    for (int pr = 0; pr < 4; ++pr) {
-      if (!P::tpair_needed(pr)) continue;
-      T v0 = T(0), v1 = T(0);
+          for (int pr = 0; pr < 4; ++pr)
+            if (P::tpair_needed(pr))
+              dmma_8x8x4(e[pr & 1][0], e[pr & 1][1],
+                         fw2[(a2_slot<P>(pr >> 1) * 2 * NBK + 2 * mt + i) * 32], v[pr][i]);
 #pragma unroll
-      for (int i = 0; i < I; ++i)
-        if (P::tpair(i) == pr) {
-          v0 += acc[i][0][0];
-          v1 += acc[i][0][1];
+        for (int nt = 0; nt < NBK; ++nt) {
+          if (nt == 1 && D1r <= 8) break;
+          double c0 = 0.0, c1 = 0.0;
+#pragma unroll
+          for (int g = 0; g < 2; ++g) {
+            if (!P::a1_needed(g)) continue;
+#pragma unroll
+            for (int j = 0; j < 2; ++j)
+              dmma_8x8x4(c0, c1, e[g][j], fw1[(g_slot<P>(g) * 2 * NBK + 2 * nt + j) * 32]);
+          }
+          T* yr = ydst + ylane + mt * 8 * n1 + nt * 8;
+          const bool in = mt * 8 + gq < D2r;
+          if (in && nt * 8 + 2 * tq < D1r) atomicAdd(yr, (T)c0);
+          if (in && nt * 8 + 2 * tq + 1 < D1r) atomicAdd(yr + 1, (T)c1);
         }
-      *reinterpret_cast<double2*>(dnw + pair_slot<P>(pr) * kWarpTile) =
-          make_double2((double)v0, (double)v1);
+      }
     }
-  };
-  // ... contracted over q2, then q1, added into y: the first block, and the
-  // others where a control range exceeds eight
-  auto flush_first = [&]() {
-    double ks[2][2];
-    flush_q2(0, ks);
-    flush_q1(0, 0, ks);
-    if (D1r > 8) flush_q1(0, 1, ks);
-  };
-  auto flush_second = [&]() {
-    if (D2r > 8) {
-      double ks[2][2];
-      flush_q2(1, ks);
-      flush_q1(1, 0, ks);
-      if (D1r > 8) flush_q1(1, 1, ks);
-    }
-  };
-  auto shift_acc = [&]() {
     --yleft;
     ydst += pstride;
 #pragma unroll
@@ -448,35 +428,6 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
         for (int k = 0; k < W - 1; ++k) acc[i][k][c] = acc[i][k + 1][c];
         acc[i][W - 1][c] = T(0);
       }
-  };
-  auto retire = [&]() {
-    __syncwarp();  // the previous plane's fragments are read
-    retire_store();
-    if (yleft > 0) {
-      __syncwarp();
-      flush_first();
-      flush_second();
-    }
-    asm volatile("" ::: "memory");
-    shift_acc();
-  };
-  // both windows move (the usual case): the two chains share their barriers and
-  // fill each other's latencies
-  auto move = [&]() {
-    cp_async_wait_all();
-    __syncwarp();
-    retire_store();
-    produce_q1();
-    __syncwarp();
-    T nw[NCOMBO][2];
-    produce_q2(nw);
-    if (yleft > 0) {
-      flush_first();
-      flush_second();
-    }
-    asm volatile("" ::: "memory");
-    shift_win(nw);
-    shift_acc();
   };
 
   auto point = [&](const T* cs, const T* row) {
@@ -530,13 +481,8 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   for (int g = ga; g < gb; ++g) {
     const int enew = __ldg(glist + 1 + min(g + NB + 2, ngrp));
     if (g > ga) {  // the segment's first windows are in place
-      const int mv = en[0] & 3;
-      if (mv == 3) {
-        move();
-      } else {
-        if (mv & 2) retire();
-        if (mv & 1) produce();
-      }
+      if (en[0] & 2) retire();
+      if (en[0] & 1) produce();
     }
     const int np = (en[1] >> 2) - (en[0] >> 2);
     const bool ok = mbar_wait_bounded_ns(smem_u32(bars) + slot * 8, parity,
@@ -581,10 +527,10 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   cp_async_wait_all();
 }
 
-template <typename T, int W, class P>
+template <typename T, int W, class P, bool WIDE>
 __global__ void __launch_bounds__(32, warp_resident(sizeof(T) == 8, P::S, W))
     mfw_kernel(const __grid_constant__ FusedArgs<T> a) {
-  mfw_body<T, W, P>(a, blockIdx.x, blockIdx.y);
+  mfw_body<T, W, P, WIDE>(a, blockIdx.x, blockIdx.y);
 }
 
 // Arguments of the CTA's patch in a multi-patch launch (patch p owns CTAs
@@ -616,7 +562,7 @@ __device__ __forceinline__ int mfw_batch_args(const FusedArgs<T>* __restrict__ a
 }
 
 // Many patches of one pattern and band width in one launch.
-template <typename T, int W, class P>
+template <typename T, int W, class P, bool WIDE>
 __global__ void __launch_bounds__(32, warp_resident(sizeof(T) == 8, P::S, W))
     mfw_batch_kernel(const FusedArgs<T>* __restrict__ args, const int32_t* __restrict__ cta0,
                      int npatch, const int64_t* __restrict__ offs, const T* xb, T* yb,
@@ -624,7 +570,7 @@ __global__ void __launch_bounds__(32, warp_resident(sizeof(T) == 8, P::S, W))
   __shared__ FusedArgs<T> sa;
   const int p = mfw_batch_args<T>(args, cta0, npatch, offs, xb, yb, skip, sa);
   if (p < 0) return;
-  mfw_body<T, W, P>(sa, (int)blockIdx.x - __ldg(cta0 + p), 0);
+  mfw_body<T, W, P, WIDE>(sa, (int)blockIdx.x - __ldg(cta0 + p), 0);
 }
 
 }  // namespace iga
