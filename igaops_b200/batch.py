@@ -144,8 +144,8 @@ class _BatchArnoldi:
 
 
 # time of a point group by band width, relative to width 4 (96^3 / 128^3 FP64
-# stiffness products: 8.4, 8.9, 11 and 19 ps per point)
-_GROUP_COST = {3: 0.95, 4: 1.0, 5: 1.25, 6: 2.2}
+# stiffness products: 8.3, 8.1, 8.6 and 16.5 ps per point)
+_GROUP_COST = {3: 1.0, 4: 1.0, 5: 1.05, 6: 2.0}
 
 
 def _joint_nseg(plans) -> List[int]:

@@ -244,32 +244,6 @@ static int64_t group_list_bytes(const iga_mf_plan* p, int dtype) {
                           : group_list_offset<float>(nq, n * step_group<float>(p->width));
 }
 
-// resident CTAs of the 2D warp-per-tile kernel: the register budget's, or what
-// shared memory holds (the weight table grows with the test rows' width)
-template <typename T>
-static int warp2_resident(const iga_mf_plan* p) {
-  auto f = [&](auto pat) {
-    using P = decltype(pat);
-    const int kw = std::min(p->rwidth, kWarpFace2);
-    switch (p->width) {
-      case 3: return WarpSmem2<T, P, 3>::total(kw);
-      case 4: return WarpSmem2<T, P, 4>::total(kw);
-      case 5: return WarpSmem2<T, P, 5>::total(kw);
-      default: return WarpSmem2<T, P, 6>::total(kw);
-    }
-  };
-  int smem;
-  switch (p->op) {
-    case IGA_OP_MASS: smem = f(Pat<2, IGA_OP_MASS, 0, 0, 0, 0>{}); break;
-    case IGA_OP_STIFF:
-      smem = p->sym ? f(Pat<2, IGA_OP_STIFF, 0, 0, 0, 1>{}) : f(Pat<2, IGA_OP_STIFF, 0, 0, 0, 0>{});
-      break;
-    case IGA_OP_GRADU_V: smem = f(Pat<2, IGA_OP_GRADU_V, 0, 0, 0, 0>{}); break;
-    default: smem = f(Pat<2, IGA_OP_U_GRADV, 0, 0, 0, 0>{});
-  }
-  return std::min(kWarpResident2, 228 * 1024 / (smem + 1024));
-}
-
 template <typename T>
 static iga_status table_warp(const iga_mf_plan* p, int64_t* elems, void* table, cudaStream_t st) {
   const int o = last_orders(p), last = p->ndim - 1;
@@ -392,6 +366,24 @@ iga_status launch_dispatch<float>(const FusedArgs<float>& a, const LaunchInfo& l
 #undef IGA_W_CASES
   set_error("no fused kernel for band width %d", li.W);
   return IGA_ERR_UNSUPPORTED;
+}
+
+static LaunchInfo launch_info(const iga_mf_plan* p, int64_t ncols, cudaStream_t st) {
+  LaunchInfo li;
+  li.ndim = p->ndim;
+  li.op = p->op;
+  li.st = p->spacetime;
+  li.tt = p->time_test;
+  li.tr = p->time_trial;
+  li.sym = p->sym;
+  li.W = p->width;
+  li.FX = p->face[0];
+  li.FY = p->ndim == 3 ? p->face[1] : 1;
+  li.NST = kStages;
+  li.ncols = ncols;
+  li.stream = st;
+  li.resident = nullptr;
+  return li;
 }
 
 // shared memory of the multi-patch kernel for one patch of a pattern
@@ -583,10 +575,22 @@ iga_status iga_mf_resident(const iga_mf_plan* plan, int dtype, int32_t* ctas) {
   if (rc) return rc;
   IGA_CHECK_ARG(dtype == IGA_F64 || dtype == IGA_F32, "dtype %d not supported", dtype);
   IGA_CHECK_ARG(ctas, "null ctas");
-  *ctas = !warp_face(plan)    ? 0
-          : plan->ndim == 3 ? warp_resident(dtype == IGA_F64, plan->nstream, plan->width)
-          : dtype == IGA_F64  ? warp2_resident<double>(plan)
-                              : warp2_resident<float>(plan);
+  *ctas = 0;
+  if (!warp_face(plan)) return IGA_OK;
+  LaunchInfo li = launch_info(plan, 1, nullptr);
+  int n = 0;
+  li.resident = &n;
+  if (dtype == IGA_F64) {
+    FusedArgs<double> a;
+    fill_args<double>(a, plan, nullptr, nullptr, nullptr);
+    rc = launch_dispatch<double>(a, li);
+  } else {
+    FusedArgs<float> a;
+    fill_args<float>(a, plan, nullptr, nullptr, nullptr);
+    rc = launch_dispatch<float>(a, li);
+  }
+  if (rc) return rc;
+  *ctas = n;
   return IGA_OK;
 }
 
@@ -730,19 +734,7 @@ iga_status iga_mf_matvec(const iga_mf_plan* plan, int dtype, const void* packed,
   for (int d = 0; d < plan->ndim; ++d) N *= plan->n[d];
   const size_t esz = dtype == IGA_F64 ? 8 : 4;
   IGA_CUDA_TRY(cudaMemsetAsync(y, 0, (size_t)N * ncols * esz, st));
-  LaunchInfo li;
-  li.ndim = plan->ndim;
-  li.op = plan->op;
-  li.st = plan->spacetime;
-  li.tt = plan->time_test;
-  li.tr = plan->time_trial;
-  li.sym = plan->sym;
-  li.W = plan->width;
-  li.FX = plan->face[0];
-  li.FY = plan->ndim == 3 ? plan->face[1] : 1;
-  li.NST = kStages;
-  li.ncols = ncols;
-  li.stream = st;
+  const LaunchInfo li = launch_info(plan, ncols, st);
   if (dtype == IGA_F64) {
     FusedArgs<double> a;
     fill_args<double>(a, plan, packed, x, y);

@@ -1324,6 +1324,7 @@ struct LaunchInfo {
   int FX, FY, NST;
   int64_t ncols;
   cudaStream_t stream;
+  int* resident;  // not null: report the kernel's resident CTAs per SM, launch nothing
 };
 
 // One object file per (dimension, element type, band width); see mf_inst.cu.

@@ -19,7 +19,7 @@ static iga_status launch_pat(const FusedArgs<T>& a, const LaunchInfo& li) {
   const dim3 grid((unsigned)(a.tiles1 * a.tiles2 * a.nseg), (unsigned)li.ncols);
   if constexpr (D == 3) {
     if (li.FX == kWarpFace && li.FY == kWarpFace) {
-      if (!a.step_table) {
+      if (!a.step_table && !li.resident) {
         set_error("3D fused kernel needs the step table of the plan (iga_mf_table)");
         return IGA_ERR_INVALID_ARG;
       }
@@ -32,8 +32,13 @@ static iga_status launch_pat(const FusedArgs<T>& a, const LaunchInfo& li) {
         return IGA_ERR_UNSUPPORTED;
       }
       static_assert(L::total <= 48 * 1024, "shared memory of a CTA (no opt-in)");
-      if (range > kWarpFace) mfw_kernel<T, W, P, true><<<grid, 32, L::total, li.stream>>>(a);
-      else mfw_kernel<T, W, P, false><<<grid, 32, N::total, li.stream>>>(a);
+      const auto kern = range > kWarpFace ? mfw_kernel<T, W, P, true> : mfw_kernel<T, W, P, false>;
+      const size_t smem = range > kWarpFace ? L::total : N::total;
+      if (li.resident) {
+        IGA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(li.resident, kern, 32, smem));
+        return IGA_OK;
+      }
+      kern<<<grid, 32, smem, li.stream>>>(a);
       IGA_LAUNCH_CHECK();
       return IGA_OK;
     }
@@ -65,7 +70,7 @@ static iga_status launch_pat(const FusedArgs<T>& a, const LaunchInfo& li) {
   } else {
     if (li.FX == kWarpFace2) {
       using L = WarpSmem2<T, P, W>;
-      if (!a.step_table) {
+      if (!a.step_table && !li.resident) {
         set_error("2D fused kernel needs the step table of the plan (iga_mf_table)");
         return IGA_ERR_INVALID_ARG;
       }
@@ -75,7 +80,13 @@ static iga_status launch_pat(const FusedArgs<T>& a, const LaunchInfo& li) {
       }
       static_assert(L::wtab + 2 * kWarpFace2 * L::nout * (int)sizeof(T) <= 48 * 1024,
                     "shared memory of a CTA (no opt-in)");
-      mfw2_kernel<T, W, P><<<grid, 32, L::total(std::min(a.RW, kWarpFace2)), li.stream>>>(a);
+      const size_t smem = L::total(std::min(a.RW, kWarpFace2));
+      if (li.resident) {
+        IGA_CUDA_TRY(cudaOccupancyMaxActiveBlocksPerMultiprocessor(li.resident,
+                                                                   mfw2_kernel<T, W, P>, 32, smem));
+        return IGA_OK;
+      }
+      mfw2_kernel<T, W, P><<<grid, 32, smem, li.stream>>>(a);
       IGA_LAUNCH_CHECK();
       return IGA_OK;
     }

@@ -2,22 +2,22 @@
 // the operator and its patterns).
 //
 // A CTA is one warp. It owns a tile of 8 x 8 quadrature pencils (directions
-// 1, 2) and a segment of direction 3; lane (ly, lx2) owns the neighbouring
-// pencils 2 lx2, 2 lx2 + 1 of row ly. Nothing is shared between warps, so the march has no CTA
+// 1, 2) and a segment of direction 3, two pencils per lane. Nothing is shared between warps, so the march has no CTA
 // barrier, a point's band values are loaded once for the whole tile, and
 // everything that belongs to the tile (pointers, counters, branches) is uniform
 // over the CTA and lives on the uniform datapath.
 //
 // The points of direction 3 are taken in groups: runs of at most kGroupPts
 // points between window moves (an element, usually). Before a group
-//   * the test window moves: the oldest accumulator plane is final; it goes to
-//     shared memory and two chains of FP64 tensor-core products (m8n8k4)
-//     contract it over q2 and q1. The first chain's result fragment is the
-//     second chain's A operand when the second contraction takes the even
-//     points of q1 in its first k-step and the odd ones in its second, so the
-//     intermediate stays in registers;
+//   * the test window moves: the oldest accumulator plane is final and two chains
+//     of FP64 tensor-core products (m8n8k4) contract it over q2 and q1;
 //   * the trial window moves: the next control plane's slab (copied one plane
-//     ahead) is contracted over directions 1 and 2.
+//     ahead) is contracted over directions 1 and 2, on the tensor cores too.
+// A lane owns the pencils (q1 = lane / 4, q2 = 2 (lane mod 4) + i), i = 0, 1: with
+// the k-steps of a product taking the even and the odd members of the contracted
+// index, the accumulators of one product are the operand of the next and the
+// window entries come out at their owners, so only the slab and the weight
+// fragments pass through shared memory.
 // At a point the coefficients mix the W-long trial dot products and the result
 // is spread over the W test accumulators. A group's coefficients are one bulk
 // copy (packed [group][tile][point][stream][pencil], padding pencils zero) with
@@ -25,19 +25,18 @@
 // march through the groups at about the same pace, so with the group outermost
 // they read one moving window of the stream instead of a page each.
 //
-// What bounds it: instruction issue and the latency of the per-group chain
-// (production, points, flush) at the residency that registers allow; FP64
-// stiffness at 2 KB of registers per lane pair of pencils runs eight warps per
-// SM and comes within 15-20 % of the measured copy bandwidth. Measured against
-// the CTA-per-tile kernel (16 x 8 tiles, shared chunks, CTA barriers; B200, CUDA
-// events, best segment count, us): FP64 stiffness 3D p3 128^3 919 -> 520
-// (2861 MB, 5.5 TB/s; 600 once the power cap lowers the SM clock to 1.7 GHz),
-// p4 96^3 576 -> 275, p5 96^3 663 -> 491; FP64 mass p3 128^3 438 -> 210, p2 96^3
-// 177 -> 85; FP32 stiffness p3 128^3 606 -> 310, p4 61 x 57 x 63 94 -> 53; FP64
-// gradu_v p2 40^3 34 -> 22; 9.5 -> 4.1 (stiffness) and 5.4 -> 1.9 (mass) warp
-// instructions per point. Four warps per CTA with a batch of fixed length cost
-// 25 % more (per-warp values in vector registers), two blocks of pencils per
-// lane gained 5 % for FP64 mass and lost 20 % for FP32 stiffness.
+// What bounds it: HBM for the stiffness (FP64 p3 128^3 2861 MB in 476 us, 6.0 TB/s,
+// until the power cap lowers the SM clock to 1.7 GHz), latency and issue of the
+// per-group chain for the mass, whose points carry eight bytes each. Against the
+// CTA-per-tile kernel (16 x 8 tiles, shared chunks, CTA barriers; B200, CUDA
+// events, best segment count, us): FP64 stiffness 3D p3 128^3 919 -> 476, p4 96^3
+// 576 -> 216, p5 96^3 663 -> 420; FP64 mass p3 128^3 438 -> 155, p2 96^3 177 -> 62;
+// FP32 stiffness p3 128^3 606 -> 268, p4 61 x 57 x 63 94 -> 46; FP64 gradu_v p2 40^3
+// 34 -> 18. On the way: plane work through shared memory (a barrier per stage, the
+// shared-memory pipe at 78 %) 525 and 214 us for the first two and four; four warps
+// per CTA with batches of fixed length 25 % slower (per-warp values in vector
+// registers); prefetching a third group into L2 and broadcasting tile constants by
+// shuffles changed nothing.
 #pragma once
 
 #include "mf_fused.cuh"
@@ -105,10 +104,10 @@ constexpr int kGroupPts = 3;
 constexpr int kWarpRing = 2;
 
 // Resident CTAs (warps) per SM that the register budget is set for. Measured at
-// 96^3 / 128^3 (us, best segment count): FP64 stiffness p3 8: 520, 12: 627
-// (spills), p4 8: 282, 12: 471; FP64 gradu_v p3 8: 170, 12: 149, p5 8: 262, 12:
-// 335; FP64 mass p2 16: 94, 20: 85, 24: 91, p5 16: 155, 20: 189; FP32 stiffness
-// p4 8: 205, 12: 172, 16: 177; FP32 mass p4 16: 85, 20: 76, 24: 80.
+// 96^3 / 128^3 (us, best segment count): FP64 stiffness p3 8: 478, 12: 523, p4 8:
+// 216, 12: 405 (spills); FP64 gradu_v p3 8: 170, 12: 124, p5 8: 262, 12: 317; FP64
+// mass p2 16: 68, 20: 62, 24: 69, p5 16: 140, 20: 148; FP32 stiffness p4 12: 148,
+// 16: 150, p5 12: 245, 16: 291; FP32 mass 20 (80 registers).
 __host__ __device__ constexpr int warp_resident(bool f64, int S, int W) {
   return f64 ? (S > 3 ? 8 : S > 1 ? (W <= 4 ? 12 : 8) : (W <= 4 ? 20 : 16)) : (S > 1 ? 12 : 20);
 }
@@ -139,10 +138,14 @@ struct WarpSmem {
   static constexpr int total = w1 + ng<P>() * NBK * 2 * 256;
 };
 
-// Asynchronous copy of one element to shared memory.
+// Asynchronous copy of one element to shared memory, where `in` holds.
 template <int BYTES>
-__device__ __forceinline__ void cp_async_elem(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;" ::"r"(dst), "l"(src), "n"(BYTES) : "memory");
+__device__ __forceinline__ void cp_async_elem(uint32_t dst, const void* src, bool in) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\t"
+      "@p cp.async.ca.shared.global [%0], [%1], %2;\n\t}" ::"r"(dst),
+      "l"(src), "n"(BYTES), "r"((uint32_t)in)
+      : "memory");
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
@@ -287,33 +290,29 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   const int64_t pstride = (int64_t)n1 * n2;  // control points per plane
   // x slab of one control plane, copied one plane ahead into the other half of
   // xs, 4 rows x 8 columns per pass (rows paired so that a half-warp's two rows
-  // fall on different banks). Rows and columns past the control range repeat its
-  // last, control points beyond the patch the patch's last: all meet zero weights.
+  // fall on different banks). Entries past the control range or the patch stay
+  // zero; they meet zero weights.
+  for (int e = lane; e < 2 * L::xhalf / E; e += 32) xs[e] = T(0);
   const int xr0 = ((lane >> 3) & 1) * 2 + (lane >> 4), xc0 = lane & 7;
-  auto xoff = [&](int r, int c) {
-    return min(min(r, C2r - 1), n2 - 1 - c2lo) * n1 + min(min(c, C1r - 1), n1 - 1 - c1lo);
-  };
-  const int xg0 = xoff(xr0, xc0), xg1 = xoff(xr0 + 4, xc0);
+  const int xrows = min(C2r, n2 - c2lo), xcols = min(C1r, n1 - c1lo);
+  const bool xin0 = xr0 < xrows && xc0 < xcols, xin1 = xr0 + 4 < xrows && xc0 < xcols;
   const T* xsrc = a.x + (int64_t)col * a.N + (int64_t)c2lo * n1 + c1lo;
   int xplane = __ldg(a.tstart[2] + qa);
   xsrc += min(xplane, n3 - 1) * pstride;
+  const int xg0 = xr0 * n1 + xc0, xg1 = xg0 + 4 * n1;
   const uint32_t xdst = smem_u32(xs) + (xr0 * XR + xc0) * E;
   int xflip = 0;  // half (bytes) that the next copy fills
   auto fetch = [&]() {
-    cp_async_elem<E>(xdst + xflip, xsrc + xg0);
-    cp_async_elem<E>(xdst + xflip + 4 * XR * E, xsrc + xg1);
+    cp_async_elem<E>(xdst + xflip, xsrc + xg0, xin0);
+    cp_async_elem<E>(xdst + xflip + 4 * XR * E, xsrc + xg1, xin1);
     if constexpr (WIDE) {
-      if (C2r > 8) {
-        cp_async_elem<E>(xdst + xflip + 8 * XR * E, xsrc + xoff(xr0 + 8, xc0));
-        cp_async_elem<E>(xdst + xflip + 12 * XR * E, xsrc + xoff(xr0 + 12, xc0));
-      }
-      if (C1r > 8) {
-        constexpr int C = 4 * L::KC - 8;  // columns 8 .. 4 KC - 1
-#pragma unroll 1
-        for (int e = lane; e < C * L::rows; e += 32)
-          cp_async_elem<E>(smem_u32(xs) + xflip + (e / C * XR + 8 + e % C) * E,
-                           xsrc + xoff(e / C, 8 + e % C));
-      }
+      for (int r = 8; r < xrows; r += 4)
+        cp_async_elem<E>(xdst + xflip + r * XR * E, xsrc + xg0 + r * n1,
+                         xr0 + r < xrows && xc0 < xcols);
+      for (int c = 8; c < xcols; c += 4)  // 8 rows x 4 columns per pass
+        for (int r = lane >> 2; r < xrows; r += 8)
+          cp_async_elem<E>(smem_u32(xs) + xflip + (r * XR + c + (lane & 3)) * E,
+                           xsrc + r * n1 + c + (lane & 3), c + (lane & 3) < xcols);
     }
     cp_async_commit();
     if (++xplane < n3) xsrc += pstride;

@@ -271,14 +271,18 @@ class FusedPlan:
         warps.  A unit costs its share of the groups plus a fixed part (set-up,
         W plane productions and flushes), about five groups; a warp with the SM
         to itself takes a group in 1 / 1.6 of the time it takes among all
-        resident ones (3D p3 128^3 mass: 1.03 against 1.6 us).  The last,
-        partly filled wave is charged at its own residency."""
+        resident ones (3D p3 128^3 mass: 1.03 against 1.6 us).  The last, partly
+        filled wave is charged at its own residency.  Warps that start together
+        do the same things at the same time, a quarter slower until they drift
+        apart: one unit's length of that is charged (128^3 mass in one segment
+        213 us, in four 154)."""
         full = _SM_COUNT * max(self.resident, 3)
 
         def cost(ns):
             units = self.tiles * ns
             waves, rest = divmod(units, full)
-            return (1.6 * waves + (1 + 0.6 * rest / full if rest else 0)) * (self.groups / ns + 5)
+            length = self.groups / ns + 5
+            return (1.6 * waves + (1 + 0.6 * rest / full if rest else 0) + 0.4) * length
 
         return sorted(range(1, max(1, min(most, self.groups // 2)) + 1), key=cost)
 
