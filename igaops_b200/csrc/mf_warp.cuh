@@ -1,11 +1,11 @@
 // Warp-per-tile form of the fused 3D matrix-free operator (see mf_fused.cuh for
 // the operator and its patterns).
 //
-// A CTA is one warp. It owns a tile of 8 x 8 quadrature pencils (directions
-// 1, 2) and a segment of direction 3, two pencils per lane. Nothing is shared between warps, so the march has no CTA
-// barrier, a point's band values are loaded once for the whole tile, and
-// everything that belongs to the tile (pointers, counters, branches) is uniform
-// over the CTA and lives on the uniform datapath.
+// A CTA is one warp. It owns a tile of 8 x 8 quadrature pencils (directions 1, 2) and
+// a segment of direction 3, two pencils per lane. Nothing is shared between warps, so
+// the march has no CTA barrier, a point's band values are loaded once for the whole
+// tile, and everything that belongs to the tile (pointers, counters, branches) is
+// uniform over the CTA and lives on the uniform datapath.
 //
 // The points of direction 3 are taken in groups: runs of at most kGroupPts
 // points between window moves (an element, usually). Before a group
@@ -183,6 +183,18 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   // ----------------------------------------------------- groups of the segment
   const int* glist = reinterpret_cast<const int*>(reinterpret_cast<const char*>(a.step_table) +
                                                   group_list_offset<T>(nq3, L::row));
+  // what depends on the tile alone is loaded before any of it is used; wide bands
+  // have no registers to hold it over the ring's prologue and load it at its use
+  int early[10];
+  if constexpr (!WIDE) {
+    early[0] = __ldg(a.tstart[0] + q1lo), early[1] = __ldg(a.tstart[0] + q1lo + w1 - 1);
+    early[2] = __ldg(a.tstart[1] + q2lo), early[3] = __ldg(a.tstart[1] + q2lo + w2 - 1);
+    early[4] = __ldg(a.wtstart[0] + q1lo), early[5] = __ldg(a.wtstart[0] + q1lo + w1 - 1);
+    early[6] = __ldg(a.wtstart[1] + q2lo), early[7] = __ldg(a.wtstart[1] + q2lo + w2 - 1);
+    early[8] = __ldg(a.tstart[0] + q1lo + min(lane >> 2, w1 - 1));
+    early[9] = __ldg(a.tstart[1] + q2lo + min(lane >> 2, w2 - 1));
+  }
+  auto tile_int = [&](int slot, const int* at) { return WIDE ? __ldg(at) : early[slot]; };
   auto entry = [&](int g) { return __shfl_sync(0xffffffffu, __ldg(glist + 1 + g), 0); };
   const int ngrp = __shfl_sync(0xffffffffu, __ldg(glist), 0);
   const int ga = (int)((int64_t)ngrp * seg / a.nseg), gb = (int)((int64_t)ngrp * (seg + 1) / a.nseg);
@@ -222,14 +234,14 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   }
 
   // ------------------------------------------------------------ tile tables
-  const int c1lo = __ldg(a.tstart[0] + q1lo);
-  const int C1r = __ldg(a.tstart[0] + q1lo + w1 - 1) - c1lo + W;
-  const int c2lo = __ldg(a.tstart[1] + q2lo);
-  const int C2r = __ldg(a.tstart[1] + q2lo + w2 - 1) - c2lo + W;
-  const int d1lo = __ldg(a.wtstart[0] + q1lo);
-  const int D1r = min(__ldg(a.wtstart[0] + q1lo + w1 - 1) + W - 1, n1 - 1) - d1lo + 1;
-  const int d2lo = __ldg(a.wtstart[1] + q2lo);
-  const int D2r = min(__ldg(a.wtstart[1] + q2lo + w2 - 1) + W - 1, n2 - 1) - d2lo + 1;
+  const int c1lo = tile_int(0, a.tstart[0] + q1lo);
+  const int C1r = tile_int(1, a.tstart[0] + q1lo + w1 - 1) - c1lo + W;
+  const int c2lo = tile_int(2, a.tstart[1] + q2lo);
+  const int C2r = tile_int(3, a.tstart[1] + q2lo + w2 - 1) - c2lo + W;
+  const int d1lo = tile_int(4, a.wtstart[0] + q1lo);
+  const int D1r = min(tile_int(5, a.wtstart[0] + q1lo + w1 - 1) + W - 1, n1 - 1) - d1lo + 1;
+  const int d2lo = tile_int(6, a.wtstart[1] + q2lo);
+  const int D2r = min(tile_int(7, a.wtstart[1] + q2lo + w2 - 1) + W - 1, n2 - 1) - d2lo + 1;
   // Weight fragments (lane = 4 gq + tq holds A[gq][tq] or B[tq][gq]), zero outside
   // the bands and the tile. A lane's pencils are (q1 = gq, q2 = 2 tq + i), so with
   // the k index of a product standing for point 2 tq + i (i = k-step) or control
@@ -241,7 +253,7 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   double* fw1 = reinterpret_cast<double*>(smem + L::w1) + lane;
   {
     const int q1 = q1lo + min(gq, w1 - 1), q2 = q2lo + min(gq, w2 - 1);
-    const int s1 = __ldg(a.tstart[0] + q1) - c1lo, s2 = __ldg(a.tstart[1] + q2) - c2lo;
+    const int s1 = tile_int(8, a.tstart[0] + q1) - c1lo, s2 = tile_int(9, a.tstart[1] + q2) - c2lo;
     auto band = [&](const T* v, int q, int k) {
       return k >= 0 && k < W ? (double)__ldg(v + (int64_t)q * W + k) : 0.0;
     };
@@ -320,13 +332,10 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
 
   T win[NCOMBO][W][2];  // trial planes at the lane's pencils
   const T* xl = xs + gq * XR + tq;
-  // the landed slab contracted over q1, then q2 (both on the tensor cores, the
-  // first product's accumulators are the second's A operand); next slab under way
-  auto produce = [&]() {
-    cp_async_wait_all();
-    __syncwarp();
-    const T* xb = xl + xflip / E;
-    xflip = L::xhalf - xflip;
+  // a slab (entry (row 8 nb + gq, column 4 kt + tq) from get) contracted over q1,
+  // then q2, both on the tensor cores, the first product's accumulators being the
+  // second's A operand; the result enters the window
+  auto contract = [&](auto&& get, auto&& then) {
     double d2[NCOMBO][2];
 #pragma unroll
     for (int c = 0; c < NCOMBO; ++c) d2[c][0] = d2[c][1] = 0.0;
@@ -338,7 +347,7 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
 #pragma unroll
       for (int kt = 0; kt < L::KC; ++kt) {
         if (kt >= 2 && C1r <= 4 * kt) break;
-        const double xv = (double)xb[8 * nb * XR + 4 * kt];
+        const double xv = (double)get(nb, kt);
         if (P::b1_needed(0)) dmma_8x8x4(d1[0][0], d1[0][1], fa1[kt * 32], xv);
         if (P::b1_needed(1)) dmma_8x8x4(d1[1][0], d1[1][1], fa1[(b1_slot<P>(1) * L::KC + kt) * 32], xv);
       }
@@ -350,7 +359,7 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
             dmma_8x8x4(d2[combo_slot<P>(c)][0], d2[combo_slot<P>(c)][1], d1[c & 1][i],
                        fb2[(b2_slot<P>(c >> 1) * 2 * NBK + 2 * nb + i) * 32]);
     }
-    fetch();
+    then();
 #pragma unroll
     for (int c = 0; c < NCOMBO; ++c)
 #pragma unroll
@@ -359,6 +368,14 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
         for (int m = 0; m < W - 1; ++m) win[c][m][i] = win[c][m + 1][i];
         win[c][W - 1][i] = (T)d2[c][i];
       }
+  };
+  // the next plane: its slab has landed, the one after it gets under way
+  auto produce = [&]() {
+    cp_async_wait_all();
+    __syncwarp();
+    const T* xb = xl + xflip / E;
+    xflip = L::xhalf - xflip;
+    contract([&](int nb, int kt) { return xb[8 * nb * XR + 4 * kt]; }, fetch);
   };
 
   T acc[I][W][2];  // test planes
@@ -471,9 +488,28 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
 
   // -------------------------------------------------------------- the march
   __syncwarp();
-  fetch();
+  if constexpr (WIDE) {
+    fetch();
 #pragma unroll 1
-  for (int k = 0; k < W; ++k) produce();
+    for (int k = 0; k < W; ++k) produce();
+  } else {
+    // The first window's planes straight from global memory, all loads at once: a
+    // segment's start was a chain of W slab copies. Mass, degree 3, 8^3 and 16^3:
+    // 10.4 -> 8.5 us; stiffness, degree 3, 48^3: 39.0 -> 37.2 us, 128^3: 476 -> 468 us
+    // (burst). Wide bands keep the copies: W x 2 more registers would spill.
+    T xi[W][2];
+#pragma unroll
+    for (int k = 0; k < W; ++k) {
+#pragma unroll
+      for (int kt = 0; kt < 2; ++kt)
+        xi[k][kt] = gq < xrows && 4 * kt + tq < xcols ? __ldg(xsrc + gq * n1 + 4 * kt + tq) : T(0);
+      if (++xplane < n3) xsrc += pstride;
+    }
+    fetch();
+#pragma unroll
+    for (int k = 0; k < W; ++k)
+      contract([&](int, int kt) { return xi[k][kt]; }, [] {});
+  }
   int slot = 0;
   uint32_t parity = 0;
 #pragma unroll 1
@@ -521,7 +557,7 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
     for (int k = 0; k < NB + 1; ++k) en[k] = en[k + 1];
     en[NB + 1] = __shfl_sync(0xffffffffu, enew, 0);
   }
-#pragma unroll 1
+#pragma unroll(WIDE ? 1 : W)
   for (int k = 0; k < W; ++k) retire();
   cp_async_wait_all();
 }
