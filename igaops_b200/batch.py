@@ -319,8 +319,8 @@ class PatchBatch:
         rows zeroed; patches with skip[p] >= 0 are left at zero."""
         if self.np == 1:
             # one patch: its own operator's launch (arguments as kernel
-            # parameters, 5-7 % faster than the multi-patch kernel).  skip is
-            # not needed: a step after convergence only fills Arnoldi columns
+            # parameters, no descriptor read at a CTA's start).  skip is not
+            # needed: a step after convergence only fills Arnoldi columns
             # beyond the converged one, which the triangular solve ignores.
             p = self.patches[0]
             (p.K64 if x.dtype == torch.float64 else p.K32).apply_into(x, y)
@@ -353,8 +353,8 @@ class PatchBatch:
 
     def precond_fp64(self, x: torch.Tensor, y: torch.Tensor):
         """y = P_p^{-1} x_p for every patch with the FP64 fast-diagonalisation
-        apply (the reference's SpaceFD.apply arithmetic in FP64, SIMT mode
-        products): one apply per patch."""
+        apply (the reference's SpaceFD.apply arithmetic in FP64, mode products
+        on the FP64 tensor cores): one apply per patch."""
         o = self.seg.offs_host
         if not hasattr(self, "_fd64_work"):
             self._fd64_work = []

@@ -1,7 +1,8 @@
 // Stiffness product of many 3D patches of any band widths in one launch: patch p
 // owns CTAs [cta0[p], cta0[p+1]) and its width picks the body. One launch per
 // width, one after the other, left the SMs idle at the end of each: six mixed
-// patches (p 2 .. 4, 20 .. 50 elements) 156 us per product in three launches.
+// patches (p 2 .. 4, 20 .. 50 elements) 156 us per product in three launches,
+// 117 in this one; 111 with the segment starts of mf_warp.cuh since.
 #include "mf_fused.cuh"
 #include "mf_warp.cuh"
 

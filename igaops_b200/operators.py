@@ -348,12 +348,12 @@ class MFOperator:
     Same arithmetic as ``BsplineOperations.compute_mf_scalar_<op>(quadrule_list,
     coefficients, x, time_ders)``; the coefficients are packed once (fused
     path) so repeated applies stream them straight from HBM.  ``kernel``:
-    "pencil" -- the pencil kernel (every fused pattern); "tile" -- the FP64
+    "pencil" -- the pencil kernel (every fused pattern; a warp per tile); "tile" -- the FP64
     tensor-core tile kernel (3D stiffness with symmetric coefficients and
     mass, band width <= 5; ``igaops_b200.tile3d``); "auto" -- with
     ``nseg="auto"``, the autotuner times both on this operator where the
     tile kernel applies and keeps the faster (cached per shape; on B200 the
-    pencil kernel wins, e.g. 3D p3 128^3 stiffness 0.91 ms against the tile
+    pencil kernel wins, e.g. 3D p3 128^3 stiffness 0.47 ms against the tile
     kernel's 1.2-1.6 ms), otherwise the pencil kernel.
     ``nseg``: the pencil kernel's segment count of the streamed direction
     (None: heuristic; "auto": timed by ``igaops_b200.tune`` on this operator
