@@ -870,7 +870,7 @@ def main(argv=None):
                 "copies": "pinned host buffers; H2D / D2H on their own streams, "
                           "overlapping the neighbouring steps' matvecs"},
         "roofline": {
-            "kernel": ("mf3d_kernel (fused stiffness, FP64)" if not stiff.tiled
+            "kernel": ("mfw_kernel (fused stiffness, FP64)" if not stiff.tiled
                        else "mf3d_tile_kernel (tensor-core tile stiffness, FP64)"),
             "bound": "hbm",
             "achieved": achieved,
