@@ -1122,7 +1122,7 @@ iga_status iga_fd_tc_workspace(const int32_t* m, int64_t* elems) {
 // igaops_b200/fastdiag.py); inv_lambda: FP32, prod(m) entries (direction 1
 // fastest); x, y: FP32 or FP64 (io_dtype), full control-point vectors; y is
 // zeroed outside the box.  work0 / work1: BF16, iga_fd_tc_workspace elements
-// each, zero-initialised once by the caller (their padding is never written).
+// each, of any content (their padding does not reach a result).
 iga_status iga_fd_apply_tc(int io_dtype, const int32_t* n, const int32_t* lo, const int32_t* m,
                            const void* const* Bfwd, const void* const* Bbwd,
                            const float* inv_lambda, const void* x, void* y, void* work0,

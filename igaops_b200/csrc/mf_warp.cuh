@@ -25,11 +25,11 @@
 // march through the groups at about the same pace, so with the group outermost
 // they read one moving window of the stream instead of a page each.
 //
-// What bounds it: HBM for the stiffness (FP64 p3 128^3 2861 MB in 476 us, 6.0 TB/s,
+// What bounds it: HBM for the stiffness (FP64 p3 128^3 2861 MB in 468 us, 6.1 TB/s,
 // until the power cap lowers the SM clock to 1.7 GHz), latency and issue of the
 // per-group chain for the mass, whose points carry eight bytes each. Against the
 // CTA-per-tile kernel (16 x 8 tiles, shared chunks, CTA barriers; B200, CUDA
-// events, best segment count, us): FP64 stiffness 3D p3 128^3 919 -> 476, p4 96^3
+// events, best segment count, us): FP64 stiffness 3D p3 128^3 919 -> 468, p4 96^3
 // 576 -> 216, p5 96^3 663 -> 420; FP64 mass p3 128^3 438 -> 155, p2 96^3 177 -> 62;
 // FP32 stiffness p3 128^3 606 -> 268, p4 61 x 57 x 63 94 -> 46; FP64 gradu_v p2 40^3
 // 34 -> 18. On the way: plane work through shared memory (a barrier per stage, the
