@@ -100,7 +100,7 @@ __global__ void __launch_bounds__(kSegThreads)
 // order of every addition is fixed by (m, block count) alone.
 __global__ void __launch_bounds__(kSegThreads)
     seg_gram_stage2(int np, const int32_t* __restrict__ blk0, int m,
-                    const double* __restrict__ partial, double* __restrict__ out, int64_t ldo) {
+                    const double* partial, double* __restrict__ out, int64_t ldo) {
   __shared__ double red[kSegThreads];
   asm volatile("griddepcontrol.wait;" ::: "memory");
   const int p = blockIdx.x;
@@ -111,7 +111,7 @@ __global__ void __launch_bounds__(kSegThreads)
   const int b0 = blk0[p], b1 = blk0[p + 1];
   double v = 0.0;
   if (g < G)
-    for (int b = b0 + g; b < b1; b += G) v += partial[(int64_t)b * m + j];
+    for (int b = b0 + g; b < b1; b += G) v += ld_dependent(partial + (int64_t)b * m + j);
   red[t] = v;
   __syncthreads();
   for (int s = G / 2; s > 0; s >>= 1) {

@@ -129,4 +129,12 @@ __device__ __forceinline__ T ldg(const T* p) {
   return __ldg(p);
 }
 
+// Load of what the grid before this one wrote, in a kernel that starts before that
+// grid has ended (griddepcontrol.wait): from L2. The non-coherent path (__ldg, or a
+// const __restrict__ pointer) is for memory that nobody writes while the kernel lives.
+template <typename T>
+__device__ __forceinline__ T ld_dependent(const T* p) {
+  return __ldcg(p);
+}
+
 }  // namespace iga

@@ -35,14 +35,14 @@ __global__ void __launch_bounds__(kDenseThreads) dense_mode_kernel(const __grid_
       const T* src = p.A + (int64_t)(r_lo + r) * p.ldr;
       double* dst = As + r * lda;
 #pragma unroll 4
-      for (int c = lane; c < K; c += 32) stage_elem(dst + c, src + c);
+      for (int c = lane; c < K; c += 32) stage_elem<true>(dst + c, src + c);
     }
   } else {
     for (int c = warp * 4 + tq; c < K; c += 4 * NW) {
       const T* src = p.A + (int64_t)r_lo * p.ldr + (int64_t)c * p.ldc;
       double* dst = As + c;
 #pragma unroll 4
-      for (int r = gq; r < mr; r += 8) stage_elem(dst + r * lda, src + (int64_t)r * p.ldr);
+      for (int r = gq; r < mr; r += 8) stage_elem<true>(dst + r * lda, src + (int64_t)r * p.ldr);
     }
   }
   for (int r = tid; r < ar; r += kDenseThreads)
@@ -57,7 +57,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_mode_kernel(const __grid_
       double* dst = Xs + n;
       if (n < bn) {
 #pragma unroll 4
-        for (int c = lane & 7; c < K; c += 8) stage_elem(dst + c * LDX, src + c);
+        for (int c = lane & 7; c < K; c += 8) stage_elem<false>(dst + c * LDX, src + c);
       } else {
         for (int c = lane & 7; c < K; c += 8) dst[c * LDX] = 0.0;
       }
@@ -69,7 +69,7 @@ __global__ void __launch_bounds__(kDenseThreads) dense_mode_kernel(const __grid_
     double* dst = Xs + n;
     if (n < bn) {
 #pragma unroll 4
-      for (int c = tid / BN; c < K; c += kDenseThreads / BN) stage_elem(dst + c * LDX, src + c * p.xc);
+      for (int c = tid / BN; c < K; c += kDenseThreads / BN) stage_elem<false>(dst + c * LDX, src + c * p.xc);
     } else {
       for (int c = tid / BN; c < K; c += kDenseThreads / BN) dst[c * LDX] = 0.0;
     }

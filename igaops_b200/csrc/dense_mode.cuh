@@ -65,10 +65,12 @@ __device__ __forceinline__ void dmma(double (&d)[2], double a, double b) {
 __device__ __forceinline__ void cp8(double* dst, const double* src) {
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(smem_u32(dst)), "l"(src) : "memory");
 }
-template <typename T>
+// CONST: of a 1D factor, constant over the apply; else of a tensor, which the product
+// before may still write when this kernel starts
+template <bool CONST, typename T>
 __device__ __forceinline__ void stage_elem(double* dst, const T* src) {
   if constexpr (sizeof(T) == 8) cp8(dst, src);
-  else *dst = (double)__ldg(src);
+  else *dst = (double)(CONST ? __ldg(src) : ld_dependent(src));
 }
 
 // acc[i] += A(row block i) X(column block) over K: R row blocks at once. A[r][c]

@@ -272,7 +272,7 @@ __device__ __forceinline__ void fd_tc_body(const TcGemm& g, const int bx) {
     const int halfc = (kchunks + 1) / 2;
     const int kc0 = (tid >> 7) ? halfc : 0, kc1 = (tid >> 7) ? kchunks : halfc;
     const bool live = row0 + r < R;
-    const uint4* __restrict__ Arow =
+    const uint4* Arow =
         reinterpret_cast<const uint4*>(g.A + (size_t)(live ? row0 + r : 0) * Kp);
     unsigned char* dst = smem_raw + (size_t)r * 16;
     // Padding is not read: it holds other products' values (the work arrays change
@@ -281,7 +281,7 @@ __device__ __forceinline__ void fd_tc_body(const TcGemm& g, const int bx) {
     const int tailc = Kt & 7 ? Kt >> 3 : -1;
     uint4 tail = make_uint4(0, 0, 0, 0);
     if (live && tailc >= kc0 && tailc < kc1) {
-      tail = __ldg(Arow + tailc);
+      tail = ld_dependent(Arow + tailc);
       uint32_t* w = reinterpret_cast<uint32_t*>(&tail);
 #pragma unroll
       for (int j = 0; j < 4; ++j)
@@ -292,7 +292,7 @@ __device__ __forceinline__ void fd_tc_body(const TcGemm& g, const int bx) {
 #pragma unroll
       for (int u = 0; u < U; ++u) {
         v[u] = make_uint4(0, 0, 0, 0);
-        if (live && k0 + u < min(kc1, Kt >> 3)) v[u] = __ldg(Arow + k0 + u);
+        if (live && k0 + u < min(kc1, Kt >> 3)) v[u] = ld_dependent(Arow + k0 + u);
       }
 #pragma unroll
       for (int u = 0; u < U; ++u)
@@ -638,7 +638,7 @@ __device__ __forceinline__ void tc_stage_w1(const TcFused& g, int i3, unsigned c
       at[u] = r < rows && kc < nkc ? kc * rows * 16 + rr * 16 : -1;
       v[u] = make_uint4(0, 0, 0, 0);
       if (rr < m2 && kc < nkc)
-        v[u] = *reinterpret_cast<const uint4*>(src + (size_t)rr * kp1 + 8 * kc);
+        v[u] = ld_dependent(reinterpret_cast<const uint4*>(src + (size_t)rr * kp1 + 8 * kc));
       uint32_t* w = reinterpret_cast<uint32_t*>(&v[u]);
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -777,7 +777,7 @@ __device__ __forceinline__ void fd_tc_line(const TcFused& g, const int bx) {
 #pragma unroll
         for (int j = 0; j < 8; ++j)
           v[u][j] = rr < R && k0 + j < m3
-                        ? *reinterpret_cast<const uint32_t*>(g.w0 + (size_t)(k0 + j) * R + rr) : 0u;
+                        ? ld_dependent(reinterpret_cast<const uint32_t*>(g.w0 + (size_t)(k0 + j) * R + rr)) : 0u;
       }
 #pragma unroll
       for (int u = 0; u < U; ++u) {

@@ -111,8 +111,8 @@ __global__ void __launch_bounds__(kDenseThreads) sptime_time_kernel(const __grid
   for (int r = warp; r < ar; r += NW)
     for (int c = lane; c < lda; c += 32) {
       if (r < mt && c < mt) {
-        stage_elem(Ar + r * lda + c, p.ur + (int64_t)r * mt + c);
-        stage_elem(Ai + r * lda + c, p.ui + (int64_t)r * mt + c);
+        stage_elem<true>(Ar + r * lda + c, p.ur + (int64_t)r * mt + c);
+        stage_elem<true>(Ai + r * lda + c, p.ui + (int64_t)r * mt + c);
       } else {
         Ar[r * lda + c] = Ai[r * lda + c] = 0.0;
       }
@@ -120,7 +120,7 @@ __global__ void __launch_bounds__(kDenseThreads) sptime_time_kernel(const __grid
   asm volatile("griddepcontrol.wait;" ::: "memory");
   for (int e = tid; e < ar * BN; e += kDenseThreads) {
     const int i = e / BN, j = e % BN;
-    if (i < mt && j < bn) stage_elem(Xs + i * LDX + j, p.x + (int64_t)i * p.ms + j0 + j);
+    if (i < mt && j < bn) stage_elem<false>(Xs + i * LDX + j, p.x + (int64_t)i * p.ms + j0 + j);
     else Xs[i * LDX + j] = 0.0;
   }
   if constexpr (sizeof(T) == 8) asm volatile("cp.async.wait_all;" ::: "memory");
