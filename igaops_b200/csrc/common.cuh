@@ -8,6 +8,7 @@
 
 #include "igab200.h"
 #include "fastdiv.cuh"
+#include "smem_optin.cuh"
 
 namespace iga {
 

@@ -177,11 +177,8 @@ static DenseTile dense_tile(int rows, int cols, int64_t N, bool two) {
 template <typename T, int BN, bool TWO>
 static iga_status launch_tile(const DenseMode<T>& p, size_t smem, bool dependent, cudaStream_t st) {
   auto kern = dense_mode_kernel<T, BN, TWO>;
-  static size_t configured = 48 * 1024;
-  if (smem > configured) {
-    IGA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    configured = 227 * 1024;
-  }
+  static SmemOptIn optin;
+  IGA_CUDA_TRY(optin.allow((const void*)kern, smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ceil_div(p.N, BN), (unsigned)ceil_div(p.rows, p.mb));
   cfg.blockDim = dim3(kDenseThreads);

@@ -888,13 +888,6 @@ __global__ void __launch_bounds__(NT)
   fd_tc_stage<NT, STAGE>(sg, (int)blockIdx.x - first, yb, zero_bytes);
 }
 
-template <int A_MODE, int O_MODE>
-static iga_status set_smem_tc(size_t smem) {
-  IGA_CUDA_TRY(cudaFuncSetAttribute(fd_tc_batch_kernel<A_MODE, O_MODE>,
-                                    cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  return IGA_OK;
-}
-
 // Launch configuration of one product: products after the first of an
 // apply overlap their launch and prologue with the previous product
 // (programmatic stream serialization; the kernels wait for it in-kernel).
@@ -919,12 +912,8 @@ template <int A_MODE, int O_MODE>
 static iga_status launch_tc_batch(const TcGemm* gs, const int32_t* cta0, int np,
                                   const int64_t* offs, int grid, size_t smem, const void* x,
                                   void* y, const int32_t* skip, cudaStream_t st, bool overlap) {
-  static size_t configured = 48 * 1024;
-  if (smem > configured) {
-    iga_status rc = set_smem_tc<A_MODE, O_MODE>(smem);
-    if (rc) return rc;
-    configured = smem;
-  }
+  static SmemOptIn optin;
+  IGA_CUDA_TRY(optin.allow((const void*)fd_tc_batch_kernel<A_MODE, O_MODE>, smem));
   TcLaunch L((unsigned)grid, smem, st, overlap);
   IGA_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, fd_tc_batch_kernel<A_MODE, O_MODE>, gs, cta0, np, offs,
                                   x, y, skip));
@@ -990,12 +979,8 @@ template <int A_MODE, int O_MODE>
 static iga_status launch_tc(const TcGemm& g, cudaStream_t st, bool overlap) {
   const size_t smem = (size_t)(128 + g.Np) * g.Kp * 2;
   auto kern = fd_tc_kernel<A_MODE, O_MODE>;
-  static size_t configured = 48 * 1024;
-  if (smem > configured) {
-    IGA_CUDA_TRY(
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+  static SmemOptIn optin;
+  IGA_CUDA_TRY(optin.allow((const void*)kern, smem));
   TcLaunch L((unsigned)(ceil_div(g.R, 128) * tc_nsplit(g.Np)), smem, st, overlap);
   IGA_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, kern, g));
   IGA_LAUNCH_CHECK();
@@ -1043,13 +1028,9 @@ static size_t tc_fused_smem_max(const TcFused& g) {
 constexpr int64_t kTcZeroPerCta = 256 * 1024;
 
 template <typename K, typename... A>
-static iga_status launch_tc_fused(K kern, size_t& configured, int threads, int64_t grid,
-                                  size_t smem, cudaStream_t st, bool overlap, A... args) {
-  if (smem > configured) {
-    IGA_CUDA_TRY(
-        cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    configured = smem;
-  }
+static iga_status launch_tc_fused(K kern, SmemOptIn& optin, int threads, int64_t grid, size_t smem,
+                                  cudaStream_t st, bool overlap, A... args) {
+  IGA_CUDA_TRY(optin.allow((const void*)kern, smem));
   TcLaunch L((unsigned)grid, smem, st, overlap, (unsigned)threads);
   IGA_CUDA_TRY(cudaLaunchKernelEx(&L.cfg, kern, args...));
   IGA_LAUNCH_CHECK();
@@ -1057,8 +1038,8 @@ static iga_status launch_tc_fused(K kern, size_t& configured, int threads, int64
 }
 template <int NT, int STAGE>
 static iga_status launch_tc_stage(const TcFused& g, int64_t zero_bytes, cudaStream_t st) {
-  static size_t configured = 48 * 1024;
-  return launch_tc_fused(fd_tc_fused_kernel<NT, STAGE>, configured, NT, tc_fused_ctas(g, STAGE),
+  static SmemOptIn optin;
+  return launch_tc_fused(fd_tc_fused_kernel<NT, STAGE>, optin, NT, tc_fused_ctas(g, STAGE),
                          tc_fused_smem(g, STAGE), st, STAGE > 0, g, zero_bytes);
 }
 template <int NT>
@@ -1082,8 +1063,8 @@ struct TcBatchArgs {
 };
 template <int NT, int STAGE>
 static iga_status launch_tc_batch_stage(const TcBatchArgs& b, int64_t zero_bytes, cudaStream_t st) {
-  static size_t configured = 48 * 1024;
-  return launch_tc_fused(fd_tc_fused_batch_kernel<NT, STAGE>, configured, NT, b.grid[STAGE], b.smem,
+  static SmemOptIn optin;
+  return launch_tc_fused(fd_tc_fused_batch_kernel<NT, STAGE>, optin, NT, b.grid[STAGE], b.smem,
                          st, STAGE > 0, b.gs, b.cta0[STAGE], b.np, b.offs, b.x, b.y, b.skip,
                          zero_bytes);
 }

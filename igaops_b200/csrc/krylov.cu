@@ -365,15 +365,13 @@ iga_status iga_gram(int dtype, int cplx, int64_t n, int m1, const void* A, int64
     // wide row sets (m1 + m2 above 2560 real / 1280 complex FP64 rows) need
     // more than the default dynamic shared-memory window even at one row
     // per tile
+    static SmemOptIn optin[3];
     if (dtype == IGA_F64 && cplx)
-      IGA_CUDA_TRY(cudaFuncSetAttribute(gram_stage1<double, true>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      IGA_CUDA_TRY(optin[0].allow((const void*)gram_stage1<double, true>, smem));
     else if (dtype == IGA_F64)
-      IGA_CUDA_TRY(cudaFuncSetAttribute(gram_stage1<double, false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      IGA_CUDA_TRY(optin[1].allow((const void*)gram_stage1<double, false>, smem));
     else
-      IGA_CUDA_TRY(cudaFuncSetAttribute(gram_stage1<float, false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      IGA_CUDA_TRY(optin[2].allow((const void*)gram_stage1<float, false>, smem));
   }
   if (dtype == IGA_F64) {
     if (cplx)
@@ -473,15 +471,13 @@ iga_status iga_combine(int dtype, int cplx, int64_t n, int m_in, const void* A, 
   if (n == 0) return IGA_OK;
   const unsigned g = grid_for(n);
   if (smem > 48 * 1024) {
+    static SmemOptIn optin[3];
     if (dtype == IGA_F64 && cplx)
-      IGA_CUDA_TRY(cudaFuncSetAttribute(combine_kernel<double, true>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      IGA_CUDA_TRY(optin[0].allow((const void*)combine_kernel<double, true>, smem));
     else if (dtype == IGA_F64)
-      IGA_CUDA_TRY(cudaFuncSetAttribute(combine_kernel<double, false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      IGA_CUDA_TRY(optin[1].allow((const void*)combine_kernel<double, false>, smem));
     else
-      IGA_CUDA_TRY(cudaFuncSetAttribute(combine_kernel<float, false>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      IGA_CUDA_TRY(optin[2].allow((const void*)combine_kernel<float, false>, smem));
   }
   if (dtype == IGA_F64) {
     if (cplx)

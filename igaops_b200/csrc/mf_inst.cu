@@ -60,12 +60,8 @@ static iga_status launch_pat(const FusedArgs<T>& a, const LaunchInfo& li) {
       return IGA_ERR_UNSUPPORTED;
     }
     auto kern = mf3d_kernel<T, FX, FY, W, P>;
-    static size_t configured = 48 * 1024;
-    if (smem > configured) {
-      IGA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem));
-      configured = smem;
-    }
+    static SmemOptIn optin;
+    IGA_CUDA_TRY(optin.allow((const void*)kern, smem));
     kern<<<grid, FX * FY, smem, li.stream>>>(a);
   } else {
     if (li.FX == kWarpFace2) {
@@ -98,12 +94,8 @@ static iga_status launch_pat(const FusedArgs<T>& a, const LaunchInfo& li) {
     }
     const size_t smem = mf2d_smem_bytes<T>(P::S, FX, NST);
     auto kern = mf2d_kernel<T, FX, W, NST, P>;
-    static size_t configured = 48 * 1024;
-    if (smem > configured) {
-      IGA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                        (int)smem));
-      configured = smem;
-    }
+    static SmemOptIn optin;
+    IGA_CUDA_TRY(optin.allow((const void*)kern, smem));
     kern<<<grid, FX, smem, li.stream>>>(a);
   }
   IGA_LAUNCH_CHECK();
@@ -160,12 +152,8 @@ static iga_status launch_pat_batch(const BatchLaunch& b, const T* x, T* y) {
     return IGA_OK;
   }
   auto kern = mf3d_batch_kernel<T, FX, FY, W, P>;
-  static size_t configured = 48 * 1024;
-  if (b.smem > configured) {
-    IGA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)b.smem));
-    configured = b.smem;
-  }
+  static SmemOptIn optin;
+  IGA_CUDA_TRY(optin.allow((const void*)kern, b.smem));
   kern<<<(unsigned)b.total_ctas, FX * FY, b.smem, b.stream>>>(
       (const FusedArgs<T>*)b.args, b.cta0, b.npatch, b.offs, x, y, b.skip);
   IGA_LAUNCH_CHECK();

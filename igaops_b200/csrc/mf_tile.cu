@@ -719,12 +719,12 @@ iga_status iga_mft_matvec(const iga_mft_plan* plan, const double* packed, int64_
     a.x = x + k * N;
     a.y = y + k * N;
     if (plan->op == IGA_OP_MASS) {
-      IGA_CUDA_TRY(cudaFuncSetAttribute(mft::mf3d_tile_kernel<IGA_OP_MASS>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      static SmemOptIn optin;
+      IGA_CUDA_TRY(optin.allow((const void*)mft::mf3d_tile_kernel<IGA_OP_MASS>, smem));
       mft::mf3d_tile_kernel<IGA_OP_MASS><<<grid, mft::NTHR, smem, st>>>(a);
     } else {
-      IGA_CUDA_TRY(cudaFuncSetAttribute(mft::mf3d_tile_kernel<IGA_OP_STIFF>,
-                                        cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      static SmemOptIn optin;
+      IGA_CUDA_TRY(optin.allow((const void*)mft::mf3d_tile_kernel<IGA_OP_STIFF>, smem));
       mft::mf3d_tile_kernel<IGA_OP_STIFF><<<grid, mft::NTHR, smem, st>>>(a);
     }
     IGA_LAUNCH_CHECK();

@@ -207,11 +207,8 @@ template <typename T>
 static iga_status launch_time(const TimeArgs<T>& a, cudaStream_t st) {
   auto kern = sptime_time_kernel<T>;
   const size_t smem = time_smem(a.mt);
-  static size_t configured = 48 * 1024;
-  if (smem > configured) {
-    IGA_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    configured = 227 * 1024;
-  }
+  static SmemOptIn optin;
+  IGA_CUDA_TRY(optin.allow((const void*)kern, smem));
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)ceil_div(a.ms, kTimeCols));
   cfg.blockDim = dim3(kDenseThreads);
