@@ -329,28 +329,35 @@ class SpaceFD:
         hit = self._dev.get(dtype)
         if hit is None:
             dev = require_cuda()
-            hit, args = [], []
+            hit = []
             for ii in range(self._nbDoFsPerNode):
                 U = [torch.from_numpy(np.ascontiguousarray(u)).to(dev, dtype)
                      for u in self._eigenvec_by_dir_space[ii]]
                 inv = torch.from_numpy(1.0 / eig[ii]).to(dev, dtype)
                 hit.append((U, inv))
-                # the call's constant arguments
-                lo, mm = self._boxes[ii]
-                arr = ctypes.c_int32 * len(mm)
-                n = arr(*[self._nonzeros_by_dir[d] for d in self._space_dirs])
-                ptrs = (ctypes.c_void_p * len(mm))(*[u.data_ptr() for u in U])
-                args.append((len(mm), n, arr(*lo), arr(*mm), ptrs, math.prod(mm)))
-            self._dev[("args", dtype)] = args
             self._dev[dtype] = hit
+        return hit
+
+    def _box_args(self, node: int):
+        """The apply's constant arguments. Sizes only: a call takes its pointers from
+        the tensors it holds, so that copies of the object, and threads that build
+        the device data at the same time, never use another's memory."""
+        hit = self._dev.get(("box", node))
+        if hit is None:
+            lo, mm = self._boxes[node]
+            arr = ctypes.c_int32 * len(mm)
+            n = arr(*[self._nonzeros_by_dir[d] for d in self._space_dirs])
+            hit = (len(mm), n, arr(*lo), arr(*mm), math.prod(mm))
+            self._dev[("box", node)] = hit
         return hit
 
     def apply_device(self, x: torch.Tensor, y: torch.Tensor, ncols: int = 1, node: int = 0,
                      work: Optional[Tuple[torch.Tensor, torch.Tensor]] = None):
         """y = P^{-1} x for one DOF-per-node block; x, y (N*ncols) with the
         column index fastest; device hot path (no host sync)."""
-        inv = self.device_data(x.dtype)[node][1]
-        ndim, n, lo, mm, ptrs, M = self._dev[("args", x.dtype)][node]
+        U, inv = self.device_data(x.dtype)[node]
+        ndim, n, lo, mm, M = self._box_args(node)
+        ptrs = (ctypes.c_void_p * ndim)(*[u.data_ptr() for u in U])
         if work is None:
             work = torch.empty((2, M * ncols), dtype=x.dtype, device=x.device)
             w0 = work.data_ptr()
