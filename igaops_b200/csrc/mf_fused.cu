@@ -142,15 +142,16 @@ __global__ void __launch_bounds__(256) mf_pack3_pm_kernel(int nq1, int nq2, int 
 
 // pack for the warp-per-tile kernels, [group][tile][point][stream][pencil], tiles
 // of F1 x F2 pencils (F2 = 1 in 2D, where nq2 = 1 and q3 counts direction 2): one
-// CTA per (row of tiles, q3); a warp walks one row of points (coalesced reads) and
-// writes its pieces into the row's tiles (pencil l1 F2 + l2), zeros beyond the grid.
+// CTA per (row of tiles, q3), both on the x axis of the grid (the others end at 65535);
+// a warp walks one row of points (coalesced reads) and writes its pieces into the row's
+// tiles (pencil l1 F2 + l2), zeros beyond the grid.
 template <typename Tin, typename Tout, int F1, int F2>
 __global__ void __launch_bounds__(256)
     mf_pack_warp_kernel(int nq1, int nq2, int nq3, int S, int tiles1, int tiles2,
                         const int32_t* __restrict__ groups, SrcRows rows,
                         const Tin* __restrict__ coefs, int64_t ld, Tout* __restrict__ packed) {
   constexpr int FT = F1 * F2;
-  const int t2 = blockIdx.x, q3 = blockIdx.y;
+  const int q3 = blockIdx.x / tiles2, t2 = blockIdx.x - q3 * tiles2;
   int lo = 0, hi = __ldg(groups);  // the group of q3
   while (hi - lo > 1) {
     const int mid = (lo + hi) >> 1;
@@ -665,9 +666,10 @@ iga_status iga_mf_pack(const iga_mf_plan* plan, int dtype_in, const void* coefs,
     const int nq2 = d3 ? plan->nq[1] : 1, nq3 = plan->nq[plan->ndim - 1];
     const int tiles1 = (int)ceil_div(plan->nq[0], plan->face[0]);
     const int tiles2 = d3 ? (int)ceil_div(nq2, kWarpFace) : 1;
-    IGA_CHECK_ARG(nq3 <= 65535, "streamed direction of %d points exceeds the grid", nq3);
+    const int64_t ctas = (int64_t)tiles2 * nq3;
+    IGA_CHECK_ARG(ctas < (1ll << 31), "%lld rows of tiles exceed the grid", (long long)ctas);
     IGA_CHECK_ARG(plan->step_table, "this face packs by the step table's groups (iga_mf_table)");
-    const dim3 grid((unsigned)tiles2, (unsigned)nq3);
+    const dim3 grid((unsigned)ctas);
     const int32_t* groups =
         (const int32_t*)((const char*)plan->step_table + group_list_bytes(plan, dtype_out));
 #define IGA_PACK(TI, TO)                                                                         \

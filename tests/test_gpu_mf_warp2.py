@@ -69,3 +69,20 @@ def test_cta_per_tile_face_2d_still_runs(cuda, monkeypatch):
     for op in ("u_v", "gradu_gradv"):
         c = coefficients(op, rl, rng)
         assert rel_err(MFOperator(rl, c, op).apply(x), OPS[op](rl, c, x)) < 1e-12
+
+
+@pytest.mark.parametrize("ndim,op", [(2, "u_v"), (2, "gradu_gradv"), (3, "u_v"), (3, "gradu_v")])
+def test_strip_of_more_points_than_a_grid_axis(cuda, ndim, op):
+    """A long strip: more than 65535 points in the streamed direction (one axis of a
+    launch grid), few in the others."""
+    from igaops_b200 import MFOperator
+
+    rng = np.random.default_rng(5)
+    rl = rules(ndim, 2, [2] * (ndim - 1) + [21850], kind="gauss")
+    assert rl[-1].nbquadpts > 65535
+    c = coefficients(op, rl, rng)
+    x = rng.standard_normal(int(np.prod([q.nbctrlpts for q in rl])))
+    oper = MFOperator(rl, c, op)
+    assert oper.fused
+    assert rel_err(oper.apply(x), OPS[op](rl, c, x)) < 1e-12
+    oper.plan.check_status()
