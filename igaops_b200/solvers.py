@@ -21,6 +21,7 @@ numpy arrays.  Numpy right-hand sides give numpy solutions.
 from __future__ import annotations
 
 import logging
+import math
 import warnings
 from dataclasses import dataclass
 from time import time
@@ -238,6 +239,20 @@ def _as_vec(y, like: torch.Tensor) -> torch.Tensor:
         like.device, like.dtype)
 
 
+def _norms_from_gram(g: np.ndarray, lengths: np.ndarray, vectors) -> Optional[List[float]]:
+    """|Z v| of each coefficient vector v from g = Z^T Z (lengths: |z_i|), or None where a
+    rounding of g could show. Each entry of g is off by at most about 1e-14 |z_i| |z_j|, so v^T g v by
+    1e-14 (sum_i |v_i| |z_i|)^2: where cancellation leaves less than 1e-8 of that sum's
+    square, the norm is no longer good to 1e-6 (it can even come out zero)."""
+    out = []
+    for v in vectors:
+        sq, bound = float(v.dot(g).dot(v)), float(np.abs(v).dot(lengths))
+        if not sq > 1e-8 * bound * bound:
+            return None
+        out.append(math.sqrt(sq))
+    return out
+
+
 # ======================================================= linear solver
 class LinearSolver:
     """Iterative solvers of the reference with device-resident vectors."""
@@ -378,9 +393,11 @@ class LinearSolver:
 
         One device-to-host read per iteration: the projections of both passes,
         the new norm and the products Z^T z.  The increment criterion's norms
-        come from the Gram matrix of Z (x = Z y, so |x|^2 = y^T Z^T Z y), so x
-        is formed once, at the end; every vector that enters A or P has zero
-        Dirichlet entries already (masked right-hand side and products)."""
+        come from the Gram matrix of Z (x = Z y, so |x|^2 = y^T Z^T Z y) where
+        that is accurate, so x is formed once, at the end; where cancellation
+        leaves too few digits (nearly dependent or badly scaled Z), x and the
+        one before it are formed and subtracted.  Every vector that enters A or P
+        has zero Dirichlet entries already (masked right-hand side and products)."""
         cm = self.convergence_manager
         ws = K.Workspace(b.device)
         n = b.shape[0]
@@ -393,6 +410,7 @@ class LinearSolver:
         m = int(cm.parameters["iteration"].reference)
         H = np.zeros((m + 1, m))
         gram = np.zeros((m, m))  # Z^T Z
+        lengths = np.zeros(m)  # |z_i|
         V = torch.empty((m + 1, n), dtype=b.dtype, device=b.device)
         Z = torch.empty((m, n), dtype=b.dtype, device=b.device)
         K.axpby(1.0 / r0, b, 0.0, V[0])
@@ -409,6 +427,7 @@ class LinearSolver:
             _check_finite_host(hv, "the Arnoldi step (operator or preconditioner output)")
             H[:it, it - 1] = hv[:it] + hv[it:2 * it]
             gram[:it, it - 1] = gram[it - 1, :it] = hv[2 * it:3 * it]
+            lengths[it - 1] = math.sqrt(hv[3 * it - 1])
             nw = float(np.sqrt(max(float(hv[3 * it]), 0.0)))
             H[it, it - 1] = nw
             if nw != 0:
@@ -421,10 +440,12 @@ class LinearSolver:
             rhs = np.zeros(it + 1)
             rhs[0] = r0
             y = lstsq(mat, rhs, rcond=None)[0]
-            dy = y - np.append(yold, 0.0)
-            g = gram[:it, :it]
-            incr = (float(np.sqrt(max(float(dy @ g @ dy), 0.0)))
-                    / (float(np.sqrt(max(float(y @ g @ y), 0.0))) + Constants.SAFEGUARD))
+            dy = y.copy()
+            dy[:-1] -= yold
+            norms = _norms_from_gram(gram[:it, :it], lengths[:it], (dy, y))
+            if norms is None:
+                norms = self._increment_norms(ws, Z, y, yold, x)
+            incr = norms[0] / (norms[1] + Constants.SAFEGUARD)
             yold = y
             r1 = float(np.linalg.norm(rhs - mat @ y))
             res.append(r1 / r0)
@@ -441,6 +462,18 @@ class LinearSolver:
         output.solution = x
         output.residual = np.asarray(res)
         return output
+
+    @staticmethod
+    def _increment_norms(ws, Z, y, yold, x) -> List[float]:
+        """|Z y - Z yold| and |Z y| of the formed vectors (x: scratch)."""
+        K.combine(Z[: len(y)], y.reshape(-1, 1), x)
+        diff = x.clone()
+        if len(yold):
+            xold = torch.empty_like(x)
+            K.combine(Z[: len(yold)], yold.reshape(-1, 1), xold)
+            K.axpby(-1.0, xold, 1.0, diff)
+        nd = torch.cat([K.gram(ws, diff, diff)[0], K.gram(ws, x, x)[0]]).cpu().numpy()
+        return [float(np.sqrt(max(float(v), 0.0))) for v in nd]
 
     # --------------------------------------------------------------- CG
     def _CG(self, Afun, b: torch.Tensor, Pfun, **kw) -> OutputArgs:
