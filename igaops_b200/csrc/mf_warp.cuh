@@ -303,7 +303,9 @@ __device__ __forceinline__ void mfw_body(const FusedArgs<T>& a, const int unit, 
   // x slab of one control plane, copied one plane ahead into the other half of
   // xs, 4 rows x 8 columns per pass (rows paired so that a half-warp's two rows
   // fall on different banks). Entries past the control range or the patch stay
-  // zero; they meet zero weights.
+  // zero; they meet zero weights. (So do entries that an output does not reach: an
+  // infinity or NaN of x or of a coefficient makes every output of the tiles whose
+  // control ranges or points hold it NaN, as it did in the 16 x 8 tiles.)
   for (int e = lane; e < 2 * L::xhalf / E; e += 32) xs[e] = T(0);
   const int xr0 = ((lane >> 3) & 1) * 2 + (lane >> 4), xc0 = lane & 7;
   const int xrows = min(C2r, n2 - c2lo), xcols = min(C1r, n1 - c1lo);

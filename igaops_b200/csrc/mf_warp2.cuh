@@ -32,9 +32,10 @@ struct WarpSmem2 {
   static constexpr int nout = kWarpFace2 + W - 1;  // outputs of a tile (unit steps)
   static constexpr int ng = (P::a1_needed(0) ? 1 : 0) + (P::a1_needed(1) ? 1 : 0);
   static constexpr int ring = 64;
+  // finished rows, with kWarpFace2 zeros before, between and after them
   static constexpr int done = ring + kWarpRing2 * slot * E;
-  static constexpr int nrow = 2 * kWarpFace2;  // a row and as many zeros
-  static constexpr int wtab = done + ng * nrow * E;
+  static constexpr int nrow = 2 * kWarpFace2;
+  static constexpr int wtab = done + (kWarpFace2 + ng * nrow) * E;
   __host__ __device__ static int total(int kw) { return wtab + (ng * kw * nout * E + 15) / 16 * 16; }
 };
 
@@ -55,7 +56,7 @@ __global__ void __launch_bounds__(32, kWarpResident2)
   const int kw = min(a.RW, kWarpFace2);
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem);
   T* ring = reinterpret_cast<T*>(smem + L::ring);
-  T* done = reinterpret_cast<T*>(smem + L::done);
+  T* done = reinterpret_cast<T*>(smem + L::done) + kWarpFace2;
   T* wtab = reinterpret_cast<T*>(smem + L::wtab);
 
   const int* glist = reinterpret_cast<const int*>(reinterpret_cast<const char*>(a.step_table) +
@@ -131,7 +132,8 @@ __global__ void __launch_bounds__(32, kWarpResident2)
   fetch();
 
   // outputs of the tile: lane o (and o + 32) reads the kw points from l0 on with
-  // the tabulated weights, zero past its band and past the tile
+  // the tabulated weights: its band, and zeros of `done` where that leaves the tile
+  // (not other points with zero weights: an infinity or NaN of theirs is not its own)
   const int d1lo = __ldg(a.wtstart[0] + q1lo);
   const int D1r = min(__ldg(a.wtstart[0] + q1lo + w1 - 1) + W - 1, n1 - 1) - d1lo + 1;
   int l0[2];
@@ -141,17 +143,18 @@ __global__ void __launch_bounds__(32, kWarpResident2)
     l0[h] = 0;
     if (o < D1r) {
       const int rs = __ldg(a.rstart[0] + d1lo + o) - q1lo;
-      l0[h] = min(max(rs, 0), kWarpFace2 - 1);
+      l0[h] = rs < 0 ? max(min(rs + a.RW - kw, 0), -kWarpFace2) : min(rs, kWarpFace2);
 #pragma unroll 1
       for (int k = 0; k < kw; ++k) {
         const int l = l0[h] + k, kk = l - rs;
-        const bool in = l < w1 && kk >= 0 && kk < a.RW;
+        const bool in = l >= 0 && l < w1 && kk >= 0 && kk < a.RW;
         const int64_t at = (int64_t)(d1lo + o) * a.RW + kk;
         if (P::a1_needed(0)) wtab[(g_slot<P>(0) * kw + k) * L::nout + o] = in ? __ldg(a.wR0[0] + at) : T(0);
         if (P::a1_needed(1)) wtab[(g_slot<P>(1) * kw + k) * L::nout + o] = in ? __ldg(a.wR1[0] + at) : T(0);
       }
     }
   }
+  done[lane - kWarpFace2] = T(0);
 #pragma unroll
   for (int g = 0; g < L::ng; ++g) done[g * L::nrow + kWarpFace2 + lane] = T(0);
 
