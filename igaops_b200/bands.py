@@ -253,10 +253,22 @@ class RuleBands:
         return hit
 
 
+def _basis_slot(q) -> dict:
+    """Cache slot of a rule's basis matrices: like factor_for it belongs to the matrices,
+    so that a rule whose basis was replaced gets new bands."""
+    slot = _CACHE.slot(q.basis[0])
+    ref = slot.get("basis1")
+    if ref is None or ref() is not q.basis[1]:
+        for key in [k for k in slot if k == "basisband" or k[0] == "basisdev"]:
+            del slot[key]
+        slot["basis1"] = weakref.ref(q.basis[1])
+    return slot
+
+
 def basis_band(q):
     """Shared band of a rule's B0 and B1, (start, [B0, B1], width, monotone, unit):
     `unit` tells whether the start advances by at most one per point."""
-    slot = _CACHE.slot(q)
+    slot = _basis_slot(q)
     hit = slot.get("basisband")
     if hit is None:
         start, vals, w, monotone = band_from([q.basis[0], q.basis[1]], unit_steps=True)
@@ -267,7 +279,7 @@ def basis_band(q):
 
 def basis_device(q, width: int) -> DeviceBand:
     """FP64 device form of basis_band padded to `width`."""
-    slot = _CACHE.slot(q)
+    slot = _basis_slot(q)
     key = ("basisdev", width, torch.cuda.current_device())
     hit = slot.get(key)
     if hit is None:

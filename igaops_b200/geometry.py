@@ -92,21 +92,21 @@ def jacobian(quadrule_list, ctrlpts) -> torch.Tensor:
     return J
 
 
-def _one_pass(quadrule_list, P: torch.Tensor) -> bool:
-    """Whether the one-pass kernel covers the patch: 3D in 3D space, bands of
-    width 2..6 whose starts move up by at most one per point.  It is the faster
-    path at every size (3D p3 64^3: 0.16 ms against 1.5 ms, 8^3: two launches
-    against thirty)."""
+def _one_pass(quadrule_list, P: torch.Tensor) -> int:
+    """Common band width where the one-pass kernel covers the patch, else 0: 3D in 3D
+    space, bands of width 2..6 whose starts move up by at most one per point.  It is
+    the faster path at every size (3D p3 64^3: 0.16 ms against 1.5 ms, 8^3: two
+    launches against thirty)."""
     if len(quadrule_list) != 3 or P.ndim != 2 or P.shape[0] != 3:
-        return False
+        return 0
     if P.shape[1] != math.prod(int(q.nbctrlpts) for q in quadrule_list):
-        return False
+        return 0
     bands = [basis_band(q) for q in quadrule_list]
-    return 2 <= max(b[2] for b in bands) <= 6 and all(b[3] and b[4] for b in bands)
+    W = max(b[2] for b in bands)
+    return W if 2 <= W <= 6 and all(b[3] and b[4] for b in bands) else 0
 
 
-def _coefficients3(quadrule_list, P: torch.Tensor, want_coef: bool):
-    W = max(basis_band(q)[2] for q in quadrule_list)
+def _coefficients3(quadrule_list, W: int, P: torch.Tensor, want_coef: bool):
     bands = [basis_device(q, W) for q in quadrule_list]
     plan = _lib.iga_mf_plan()
     plan.ndim, plan.width = 3, W
@@ -135,8 +135,9 @@ def precompute_coefficients(quadrule_list, ctrlpts, stiffness: bool = True,
     ``"mass"`` (Nq,) = det J, both float64 on the device.
     """
     P = to_device(ctrlpts, torch.float64)
-    if _one_pass(quadrule_list, P):
-        det, coef = _coefficients3(quadrule_list, P, want_coef=stiffness)
+    W = _one_pass(quadrule_list, P)
+    if W:
+        det, coef = _coefficients3(quadrule_list, W, P, want_coef=stiffness)
     else:
         J = jacobian(quadrule_list, P)
         det, _, coef = _pointwise(J, want_inv=False, want_coef=stiffness, want_det=True)
