@@ -56,11 +56,18 @@ def _save():
             pass
 
 
+# Entries of a kept file belong to the kernels that they were timed on: raised when the
+# pencil or tile kernels change what the best choice is.
+_KERNELS = "warp-per-tile 1"
+
+
 def shape_key(plan) -> str:
-    """Problem shape of a fused plan (what the best launch shape depends on)."""
+    """Problem shape of a fused plan and the kernel form (what the best launch shape
+    depends on): sizes, tile face, point groups of the streamed direction."""
     return "|".join(str(v) for v in (
         plan.ndim, plan.op, plan.st, plan.tt, plan.tr, int(plan.sym), str(plan.dtype)[6:],
-        plan.W, *plan.n, *plan.nq, torch.cuda.get_device_name()))
+        plan.W, *plan.n, *plan.nq, *plan.P.face, plan.groups, _KERNELS,
+        torch.cuda.get_device_name()))
 
 
 def candidates(plan) -> Iterable[int]:
