@@ -144,7 +144,8 @@ class _BatchArnoldi:
 
 
 # time of a point group by band width, relative to width 4 (96^3 / 128^3 FP64
-# stiffness products: 8.3, 8.1, 8.6 and 16.5 ps per point)
+# stiffness products: 8.3, 8.1, 8.6 and 16.5 ps per point; FP32 launches use them too,
+# where width 6 measured 1.65)
 _GROUP_COST = {3: 1.0, 4: 1.0, 5: 1.05, 6: 2.0}
 
 

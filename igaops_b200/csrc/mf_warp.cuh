@@ -28,8 +28,8 @@
 // What bounds it: HBM for the stiffness (FP64 p3 128^3 2861 MB in 468 us, 6.1 TB/s,
 // until the power cap lowers the SM clock to 1.7 GHz), latency and issue of the
 // per-group chain for the mass, whose points carry eight bytes each. Against the
-// CTA-per-tile kernel (16 x 8 tiles, shared chunks, CTA barriers; B200, CUDA
-// events, best segment count, us): FP64 stiffness 3D p3 128^3 919 -> 468, p4 96^3
+// CTA-per-tile kernel (16 x 8 tiles, shared chunks, CTA barriers; B200, us a launch
+// with the clearing of y, back to back, best segment count): FP64 stiffness 3D p3 128^3 919 -> 468, p4 96^3
 // 576 -> 216, p5 96^3 663 -> 420; FP64 mass p3 128^3 438 -> 155, p2 96^3 177 -> 62;
 // FP32 stiffness p3 128^3 606 -> 268, p4 61 x 57 x 63 94 -> 46; FP64 gradu_v p2 40^3
 // 34 -> 18. On the way: plane work through shared memory (a barrier per stage, the
@@ -97,7 +97,9 @@ __host__ __device__ constexpr int b2_slot(int b) {
   return (b == 1 && b2_needed<P>(0)) ? 1 : 0;
 }
 
-// Points per group: the elements of a type-2 rule have three.
+// Points per group: the elements of a type-2 rule have three. (Groups of three are
+// unrolled; the groups of two that Gauss rules of degrees 3 and 4 have take a loop, whose
+// cost was not timed apart.)
 constexpr int kGroupPts = 3;
 
 // Groups in the coefficient ring.
@@ -107,7 +109,8 @@ constexpr int kWarpRing = 2;
 // 96^3 / 128^3 (us, best segment count): FP64 stiffness p3 8: 478, 12: 523, p4 8:
 // 216, 12: 405 (spills); FP64 gradu_v p3 8: 170, 12: 124, p5 8: 262, 12: 317; FP64
 // mass p2 16: 68, 20: 62, 24: 69, p5 16: 140, 20: 148; FP32 stiffness p4 12: 148,
-// 16: 150, p5 12: 245, 16: 291; FP32 mass 20 (80 registers).
+// 16: 150, p5 12: 245, 16: 291; FP32 mass 20 (80 registers). FP64 stiffness of widths 3
+// and 6 takes width 4's and 5's (not timed by themselves).
 __host__ __device__ constexpr int warp_resident(bool f64, int S, int W) {
   return f64 ? (S > 3 ? 8 : S > 1 ? (W <= 4 ? 12 : 8) : (W <= 4 ? 20 : 16)) : (S > 1 ? 12 : 20);
 }

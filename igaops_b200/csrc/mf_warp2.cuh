@@ -9,7 +9,7 @@
 // the segments are short (the wave model decides) and nothing waits for another
 // warp. Against the CTA-per-tile kernel (128 pencils, two CTA barriers and a band
 // lookup per point, segments of 48 points), B200, us a whole call: FP64 stiffness
-// p3 64^2 58 -> 15 (launch-bound), p5 301 x 283 67 -> 29, p3 1000^2 176 -> 90,
+// p3 64^2 58 -> 13 (launch-bound), p5 301 x 283 67 -> 28, p3 1000^2 176 -> 90,
 // FP32 p3 128^2 48 -> 15, FP64 mass p4 320^2 54 -> 19.
 #pragma once
 

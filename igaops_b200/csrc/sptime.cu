@@ -226,7 +226,7 @@ static iga_status launch_time(const TimeArgs<T>& a, cudaStream_t st) {
 // The apply on y (already zero) where the time vectors fit shared memory: space
 // products, the time kernel, space products back; up to two space directions the
 // first product gathers the box and the last scatters it. sdim = 2: 5 launches
-// instead of 13 (2D p3 24^2 x 24: 86 -> 28 us a call).
+// instead of 13 (2D p3 24^2 x 24: 134 -> 27 us a call).
 template <typename T>
 static iga_status sptime_fused(int sdim, const int32_t* n, const int32_t* lo, const int32_t* m,
                                const void* const* U, TimeArgs<T> ta, const T* x, T* y, T* work0,
