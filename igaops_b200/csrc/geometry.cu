@@ -105,8 +105,8 @@ __global__ void __launch_bounds__(256) geometry_kernel(int64_t nq, int M,
 // points. J is square, so with its cofactors K (J^{-1} = K^T / det J)
 // C_ij = K_i . K_j / |det J|: no product J^T J, whose condition number is squared.
 // Rounding: directions are summed in the order 2, 1, 3 (the products: 3, 2, 1). Against
-// extended precision both orders are off by 9.1e-15 (p3 64^3, relative to the largest
-// coefficient); two FP64 results of different order differ by about as much.
+// extended precision both are off by 6.5e-15 (p3 64^3, 64 000 points, relative 2-norm of
+// C); two FP64 results of different order differ by 8.9e-15.
 //
 // A warp owns 32 consecutive points of direction 1 at one point of direction 2
 // and marches along a segment of direction 3: lane = point, with the trial

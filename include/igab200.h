@@ -179,10 +179,10 @@ iga_status iga_mf_resident(const iga_mf_plan* plan, int dtype, int32_t* ctas);
  * point holding its trial band values (B0, B1) and test band values (W0^T,
  * W1^T), each padded to 16 bytes; faces (8, 8) and (32, 1): only the orders the
  * operator reads, then the list of point groups between window moves (iga_mf_pack reads
- * it); other faces: all four, then the two band starts.  With table == NULL
- * only *elems is returned; otherwise the rows are written to `table`
- * (caller-owned, *elems elements of `dtype`).  plan->step_table must point
- * to it before iga_mf_matvec. */
+ * it, for a dtype_out that equals `dtype`); other faces: all four, then the two band
+ * starts.  With table == NULL only *elems is returned; otherwise the rows are written
+ * to `table` (caller-owned, *elems elements of `dtype`).  plan->step_table must point
+ * to it before iga_mf_matvec, with faces (8, 8) and (32, 1) also before iga_mf_pack. */
 iga_status iga_mf_table(const iga_mf_plan* plan, int dtype, int64_t* elems,
                         void* table, iga_stream stream);
 
